@@ -52,6 +52,43 @@ __device__ __forceinline__ T dir_value(const DirFaces<T> &F, int i, int j, int k
     return F.face[5][((size_t)i * F.ny + j) * F.S + d];
 }
 
+// The face values along a line of `axis` that lies wholly on a face of another
+// axis: the value of row q is p[q * step]. (i, j, k) is any voxel of the line;
+// its coordinate along `axis` is not read.
+template <typename T>
+struct FaceRun {
+    const T *p;
+    size_t step;
+};
+template <typename T>
+__device__ __forceinline__ FaceRun<T> face_run(const DirFaces<T> &F, int axis, int i, int j, int k, int d) {
+    if (axis != 0 && (i == 0 || i == F.nx - 1)) {  // x face: [ny][nz][S]
+        const T *f = i == 0 ? F.face[0] : F.face[1];
+        return axis == 1 ? FaceRun<T>{f + (size_t)k * F.S + d, (size_t)F.nz * F.S}
+                         : FaceRun<T>{f + (size_t)j * F.nz * F.S + d, (size_t)F.S};
+    }
+    if (axis != 1 && (j == 0 || j == F.ny - 1)) {  // y face: [nx][nz][S]
+        const T *f = j == 0 ? F.face[2] : F.face[3];
+        return axis == 0 ? FaceRun<T>{f + (size_t)k * F.S + d, (size_t)F.nz * F.S}
+                         : FaceRun<T>{f + (size_t)i * F.nz * F.S + d, (size_t)F.S};
+    }
+    const T *f = k == 0 ? F.face[4] : F.face[5];  // z face: [nx][ny][S]
+    return axis == 0 ? FaceRun<T>{f + (size_t)j * F.S + d, (size_t)F.ny * F.S}
+                     : FaceRun<T>{f + (size_t)i * F.ny * F.S + d, (size_t)F.S};
+}
+// Rows [q0, q1) of a face run into shared memory, row q at dst[q * stride], by
+// asynchronous element copies (no registers, any number in flight); the caller
+// waits for them with cp_wait<0>.
+template <typename T>
+__device__ __forceinline__ void face_run_copy(const FaceRun<T> &r, T *dst, int stride, int q0, int q1) {
+    const T *src = r.p + (size_t)q0 * r.step;
+    unsigned s = (unsigned)__cvta_generic_to_shared(dst + (size_t)q0 * stride);
+#pragma unroll 4
+    for (int q = q0; q < q1; ++q, src += r.step, s += (unsigned)stride * (unsigned)sizeof(T))
+        cp_async_s<sizeof(T)>(s, src);
+    cp_commit();
+}
+
 __device__ __forceinline__ bool on_active_face(unsigned m, int i, int j, int k, int nx, int ny, int nz) {
     return ((m & 1u) && i == 0) || ((m & 2u) && i == nx - 1) || ((m & 4u) && j == 0) ||
            ((m & 8u) && j == ny - 1) || ((m & 16u) && k == 0) || ((m & 32u) && k == nz - 1);

@@ -32,7 +32,7 @@ namespace bfb {
 // per SM instead of 17. Large grids are bound by shared memory and do not
 // change; many small envs stepped side by side do (256 grids of edges 32-160
 // stepped one env at a time: 6.70 -> 6.35 ms per step).
-template <typename T, bool FUSE_PRE, bool BULK>
+template <typename T, bool FUSE_PRE, bool BULK, bool DIR>
 __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 : 1)
     sweep_strided_tma_kernel(const __grid_constant__ CUtensorMap map, const __grid_constant__ CUtensorMap map_out,
                              SweepArgs<T> a, StridedGeom g, int crow) {
@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 : 1)
         fence_mbar_init();
     }
     __syncwarp();
-    strided_tma_tile<T, FUSE_PRE, BULK>(&map, &map_out, a, g, crow, tile, wbase, 0u);
+    strided_tma_tile<T, FUSE_PRE, BULK, DIR>(&map, &map_out, a, g, crow, tile, wbase, 0u);
 }
 
 // ---------------------------------------------------------------------------
@@ -140,8 +140,9 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 : 1) sweep_contig_tma_
 // constant (1 to 6, 8), 0 otherwise; every lane owns at most one line
 // (S <= 32 gives R = 32/S rows per warp).
 // ---------------------------------------------------------------------------
-template <typename T, int SC>
-__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 : 1) sweep_contig_pipe_kernel(SweepArgs<T> a, ContigGeom g, int kc) {
+template <typename T, int SC, bool DIR>
+__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 : 1)
+    sweep_contig_pipe_kernel(SweepArgs<T> a, ContigGeom g, int kc) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -159,7 +160,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 : 1) sweep_contig_pipe
         fence_mbar_init();
     }
     __syncwarp();
-    contig_pipe_tile<T, SC>(a, g, kc, tile, wbase, 0u);
+    contig_pipe_tile<T, SC, DIR>(a, g, kc, tile, wbase, 0u);
 }
 
 // ---------------------------------------------------------------------------
@@ -203,11 +204,13 @@ int launch_strided_tma(const SweepArgs<T> &a, const StridedGeom &g_in, const CUt
     const unsigned blocks = (unsigned)((tiles + warps - 1) / warps);
     const size_t smem = wb * warps;
     if (fuse_pre && a.bulk.on)
-        sweep_strided_tma_kernel<T, true, true><<<blocks, warps * 32, smem, s>>>(*map, *map_out, a, g, crow);
-    else if (fuse_pre)
-        sweep_strided_tma_kernel<T, true, false><<<blocks, warps * 32, smem, s>>>(*map, *map_out, a, g, crow);
+        sweep_strided_tma_kernel<T, true, true, true><<<blocks, warps * 32, smem, s>>>(*map, *map_out, a, g, crow);
+    else if (fuse_pre && a.dir.any)
+        sweep_strided_tma_kernel<T, true, false, true><<<blocks, warps * 32, smem, s>>>(*map, *map_out, a, g, crow);
+    else if (a.dir.any)
+        sweep_strided_tma_kernel<T, false, false, true><<<blocks, warps * 32, smem, s>>>(*map, *map_out, a, g, crow);
     else
-        sweep_strided_tma_kernel<T, false, false><<<blocks, warps * 32, smem, s>>>(*map, *map_out, a, g, crow);
+        sweep_strided_tma_kernel<T, false, false, false><<<blocks, warps * 32, smem, s>>>(*map, *map_out, a, g, crow);
     BFB_CUDA(cudaGetLastError());
     return BFB_OK;
 }
@@ -227,16 +230,22 @@ int launch_contig_tma(const SweepArgs<T> &a, const ContigGeom &g, int warps, cud
         for (int v = a.S * eb; v % 2 == 0 && q > 1; v /= 2) q /= 2;  // q = 16 / gcd(16, S*elem)
         int kc = (g.nz + chunks - 1) / chunks;
         kc = (kc + q - 1) / q * q;
+#define BFB_PIPE(SC)                                                                                  \
+    do {                                                                                              \
+        if (a.dir.any) sweep_contig_pipe_kernel<T, SC, true><<<blocks, warps * 32, smem, s>>>(a, g, kc); \
+        else sweep_contig_pipe_kernel<T, SC, false><<<blocks, warps * 32, smem, s>>>(a, g, kc);       \
+    } while (0)
         switch (a.S) {
-        case 1: sweep_contig_pipe_kernel<T, 1><<<blocks, warps * 32, smem, s>>>(a, g, kc); break;
-        case 2: sweep_contig_pipe_kernel<T, 2><<<blocks, warps * 32, smem, s>>>(a, g, kc); break;
-        case 3: sweep_contig_pipe_kernel<T, 3><<<blocks, warps * 32, smem, s>>>(a, g, kc); break;
-        case 4: sweep_contig_pipe_kernel<T, 4><<<blocks, warps * 32, smem, s>>>(a, g, kc); break;
-        case 5: sweep_contig_pipe_kernel<T, 5><<<blocks, warps * 32, smem, s>>>(a, g, kc); break;
-        case 6: sweep_contig_pipe_kernel<T, 6><<<blocks, warps * 32, smem, s>>>(a, g, kc); break;
-        case 8: sweep_contig_pipe_kernel<T, 8><<<blocks, warps * 32, smem, s>>>(a, g, kc); break;
-        default: sweep_contig_pipe_kernel<T, 0><<<blocks, warps * 32, smem, s>>>(a, g, kc); break;
+        case 1: BFB_PIPE(1); break;
+        case 2: BFB_PIPE(2); break;
+        case 3: BFB_PIPE(3); break;
+        case 4: BFB_PIPE(4); break;
+        case 5: BFB_PIPE(5); break;
+        case 6: BFB_PIPE(6); break;
+        case 8: BFB_PIPE(8); break;
+        default: BFB_PIPE(0); break;
         }
+#undef BFB_PIPE
     } else {
         sweep_contig_tma_kernel<T><<<blocks, warps * 32, smem, s>>>(a, g);
     }
@@ -258,31 +267,32 @@ static void opt_in_tma(K k) {
     cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
 }
 
+template <typename T, int SC>
+static void opt_in_pipe() {
+    opt_in_tma(sweep_contig_pipe_kernel<T, SC, true>);
+    opt_in_tma(sweep_contig_pipe_kernel<T, SC, false>);
+}
+
+template <typename T>
+static void opt_in_tma_all() {
+    opt_in_tma(sweep_strided_tma_kernel<T, true, true, true>);
+    opt_in_tma(sweep_strided_tma_kernel<T, true, false, true>);
+    opt_in_tma(sweep_strided_tma_kernel<T, false, false, true>);
+    opt_in_tma(sweep_strided_tma_kernel<T, false, false, false>);
+    opt_in_pipe<T, 1>();
+    opt_in_pipe<T, 2>();
+    opt_in_pipe<T, 3>();
+    opt_in_pipe<T, 4>();
+    opt_in_pipe<T, 5>();
+    opt_in_pipe<T, 6>();
+    opt_in_pipe<T, 8>();
+    opt_in_pipe<T, 0>();
+    opt_in_tma(sweep_contig_tma_kernel<T>);
+}
+
 void tma_prepare_device() {
-    opt_in_tma(sweep_strided_tma_kernel<double, true, true>);
-    opt_in_tma(sweep_strided_tma_kernel<double, true, false>);
-    opt_in_tma(sweep_strided_tma_kernel<double, false, false>);
-    opt_in_tma(sweep_strided_tma_kernel<float, true, true>);
-    opt_in_tma(sweep_strided_tma_kernel<float, true, false>);
-    opt_in_tma(sweep_strided_tma_kernel<float, false, false>);
-    opt_in_tma(sweep_contig_pipe_kernel<double, 1>);
-    opt_in_tma(sweep_contig_pipe_kernel<double, 2>);
-    opt_in_tma(sweep_contig_pipe_kernel<double, 3>);
-    opt_in_tma(sweep_contig_pipe_kernel<double, 4>);
-    opt_in_tma(sweep_contig_pipe_kernel<double, 5>);
-    opt_in_tma(sweep_contig_pipe_kernel<double, 6>);
-    opt_in_tma(sweep_contig_pipe_kernel<double, 8>);
-    opt_in_tma(sweep_contig_pipe_kernel<double, 0>);
-    opt_in_tma(sweep_contig_pipe_kernel<float, 1>);
-    opt_in_tma(sweep_contig_pipe_kernel<float, 2>);
-    opt_in_tma(sweep_contig_pipe_kernel<float, 3>);
-    opt_in_tma(sweep_contig_pipe_kernel<float, 4>);
-    opt_in_tma(sweep_contig_pipe_kernel<float, 5>);
-    opt_in_tma(sweep_contig_pipe_kernel<float, 6>);
-    opt_in_tma(sweep_contig_pipe_kernel<float, 8>);
-    opt_in_tma(sweep_contig_pipe_kernel<float, 0>);
-    opt_in_tma(sweep_contig_tma_kernel<double>);
-    opt_in_tma(sweep_contig_tma_kernel<float>);
+    opt_in_tma_all<double>();
+    opt_in_tma_all<float>();
 }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no libcuda link).
@@ -352,7 +362,7 @@ bool make_sweep_tensor_map_rows(CUtensorMap *out, void *field, int elem, int axi
 int strided_tile_lines(int n, int elem, int chunks) {
     if (elem != 8) return 32;
     if (chunks < 1) chunks = 1;
-    const void *kernel = (const void *)sweep_strided_tma_kernel<double, false, false>;
+    const void *kernel = (const void *)sweep_strided_tma_kernel<double, false, false, false>;
     auto resident = [&](int w) -> long long {  // lines per SM at width w (0: does not fit)
         const int crow = strided_box_rows(n, chunks, w, elem);
         const size_t wb = strided_tma_warp_bytes(n, crow, elem, w);

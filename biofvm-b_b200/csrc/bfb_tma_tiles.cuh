@@ -15,7 +15,15 @@ namespace bfb {
 // wait ran out; flush(ch) writes row group ch back once its rows are final
 // (the back substitution finishes the groups from the last to the first).
 // Returns false when a wait ran out.
-template <typename T, bool FUSE_PRE, bool BULK, int RS, typename WAIT, typename FLUSH>
+// DIR: whether any face is active. Without one the face code is compiled out.
+// Face values are global reads of about a microsecond each, so none is on a
+// line's chain: the two end values are read while the tile's copies are in
+// flight, and a column that lies wholly on a face is not solved but filled by
+// asynchronous element copies while its neighbours run the elimination. Read
+// row by row instead, the tiles on a face took ten times the others' time and
+// were every sweep's tail (200^3 x 8 FP32, x faces of one substrate: y 194 ->
+// 101 us, z 169 -> 100 us; 75^3 x 1 FP64, all faces: step 78 -> 31 us).
+template <typename T, bool FUSE_PRE, bool BULK, bool DIR, int RS, typename WAIT, typename FLUSH>
 __device__ __forceinline__ bool strided_solve(const SweepArgs<T> &a, const StridedGeom &g, int crow, int slab,
                                               long long col0, T *__restrict__ col, WAIT wait, FLUSH flush) {
     constexpr int rs = RS;  // a compile-time row stride keeps the row loops free of address arithmetic
@@ -36,7 +44,7 @@ __device__ __forceinline__ bool strided_solve(const SweepArgs<T> &a, const Strid
     const StridedColumn col_at = strided_column(a, g, slab, cl);
     const bool valid = col_at.real;
     const int d = col_at.d, ci = col_at.ci, cj = col_at.cj, ck = col_at.ck;
-    const unsigned m = (a.dir.any && valid) ? a.dir.mask[d] : 0u;
+    const unsigned m = (DIR && a.dir.any && valid) ? a.dir.mask[d] : 0u;
     bool col_dir, lo_dir, hi_dir;
     if (g.axis == 0) {
         col_dir = ((m & 4u) && cj == 0) || ((m & 8u) && cj == a.ny - 1) || ((m & 16u) && ck == 0) ||
@@ -52,6 +60,8 @@ __device__ __forceinline__ bool strided_solve(const SweepArgs<T> &a, const Strid
     auto vox_dir = [&](int mm) -> T {
         return g.axis == 0 ? dir_value(a.dir, mm, cj, ck, d) : dir_value(a.dir, ci, mm, ck, d);
     };
+    // the end rows' face values, read while the tile's copies are in flight
+    const T g_lo = lo_dir ? vox_dir(0) : T(0), g_hi = hi_dir ? vox_dir(n - 1) : T(0);
     const T *bA = nullptr, *bB = nullptr;
     if constexpr (BULK) {
         bA = a.bulk.A + (size_t)slab * g.slab_stride + cl;
@@ -71,7 +81,8 @@ __device__ __forceinline__ bool strided_solve(const SweepArgs<T> &a, const Strid
     // a line's input row after the step's leading Dirichlet
     auto xin = [&](int q) -> T {
         T x = load(q);
-        if (FUSE_PRE && ((q == 0 && lo_dir) || (q == n - 1 && hi_dir))) x = vox_dir(q);
+        if (FUSE_PRE && q == n - 1 && hi_dir) x = g_hi;
+        if (FUSE_PRE && q == 0 && lo_dir) x = g_lo;
         return x;
     };
 
@@ -80,26 +91,31 @@ __device__ __forceinline__ bool strided_solve(const SweepArgs<T> &a, const Strid
     const int ref_ch = rref / crow;
     for (int ch = 0; ch <= ref_ch; ++ch)
         if (!wait(ch)) return false;
-    col[0] = L.first(xin(0), xin(rref));
+    if (!col_dir) col[0] = L.first(xin(0), xin(rref));
     int r = 1;
     auto st_col = [&](int q, T v) { col[q * rs] = v; };
     for (int ch = 0; ch < nch; ++ch) {
         if (ch > ref_ch && !wait(ch)) return false;
+        if (col_dir) {  // the whole column lies on an active face of another axis: it takes the face's values
+            face_run_copy(face_run(a.dir, g.axis, ci, cj, ck, d), col, rs, ch * crow, min(n, (ch + 1) * crow));
+            continue;
+        }
         const int rend = min(n - 1, (ch + 1) * crow);
         const int hend = min(rend, m0);
         r = head_forward(L, r, hend, load, st_col);
         r = tail_forward(L, r, rend, load, st_col);
     }
-    if (n > 1) {
+    if (n > 1 && !col_dir) {
         T x = load(n - 1);
-        if (FUSE_PRE && hi_dir) x = vox_dir(n - 1);
+        if (FUSE_PRE && hi_dir) x = g_hi;
         L.template fwd<false>(x, n - 1);
     }
 
     // ---- back substitution into the tile; each finished row group is flushed
-    {
+    if (!col_dir) {
         T y = L.out_last();
-        if (hi_dir || (lo_dir && n == 1)) y = vox_dir(n - 1);
+        if (lo_dir && n == 1) y = g_lo;
+        if (hi_dir) y = g_hi;
         col[(n - 1) * rs] = y;
     }
     const int tl = max(m0, 1);
@@ -107,17 +123,19 @@ __device__ __forceinline__ bool strided_solve(const SweepArgs<T> &a, const Strid
     r = n - 2;
     for (int ch = nch - 1; ch >= 0; --ch) {
         const int rlo = ch * crow;
-        const int tstop = max(rlo, tl);
-        r = tail_backward(L, r, tstop, ld_col, st_col);
-        const int hstop = max(rlo, 1);
-        r = head_backward(L, r, hstop, ld_col, st_col);
-        if (rlo == 0 && n > 1) {
-            T y = L.template bwd<false>(col[0], 0);
-            if (lo_dir) y = vox_dir(0);
-            col[0] = y;
+        if (col_dir) {
+            cp_wait<0>();  // the face values have landed
+        } else {
+            const int tstop = max(rlo, tl);
+            r = tail_backward(L, r, tstop, ld_col, st_col);
+            const int hstop = max(rlo, 1);
+            r = head_backward(L, r, hstop, ld_col, st_col);
+            if (rlo == 0 && n > 1) {
+                T y = L.template bwd<false>(col[0], 0);
+                if (lo_dir) y = g_lo;
+                col[0] = y;
+            }
         }
-        if (col_dir)  // the whole column lies on an active face of another axis
-            for (int q = rlo; q < min(n, rlo + crow); ++q) col[q * rs] = vox_dir(q);
         flush(ch);
     }
     return true;
@@ -128,7 +146,7 @@ __device__ __forceinline__ bool strided_solve(const SweepArgs<T> &a, const Strid
 // tile). The mbarriers are initialised by the caller; row group ch waits for
 // parity bit ch of `phase`, and every call completes one phase of each of
 // its row groups. Returns false (error flag set) when a bounded wait ran out.
-template <typename T, bool FUSE_PRE, bool BULK, int TW>
+template <typename T, bool FUSE_PRE, bool BULK, bool DIR, int TW>
 __device__ __forceinline__ bool strided_tma_tile_w(const CUtensorMap *map, const CUtensorMap *map_out,
                                                    const SweepArgs<T> &a, const StridedGeom &g, int crow,
                                                    long long tile, unsigned char *wbase, unsigned phase) {
@@ -161,29 +179,30 @@ __device__ __forceinline__ bool strided_tma_tile_w(const CUtensorMap *map, const
             bulk_commit();
         }
     };
-    if (!strided_solve<T, FUSE_PRE, BULK, TW>(a, g, crow, slab, col0, sm + lane, wait, flush)) return false;
+    if (!strided_solve<T, FUSE_PRE, BULK, DIR, TW>(a, g, crow, slab, col0, sm + lane, wait, flush)) return false;
     if (lane == 0) bulk_wait_read_all();  // the tile must outlive the stores' reads
     __syncwarp();
     return true;
 }
 
 // The tile at the geometry's width: 32 lines, or kNarrowLinesF64 for FP64.
-template <typename T, bool FUSE_PRE, bool BULK>
+template <typename T, bool FUSE_PRE, bool BULK, bool DIR = true>
 __device__ __forceinline__ bool strided_tma_tile(const CUtensorMap *map, const CUtensorMap *map_out,
                                                  const SweepArgs<T> &a, const StridedGeom &g, int crow, long long tile,
                                                  unsigned char *wbase, unsigned phase) {
     if constexpr (sizeof(T) == 8) {
         if (g.tw == kNarrowLinesF64)
-            return strided_tma_tile_w<T, FUSE_PRE, BULK, kNarrowLinesF64>(map, map_out, a, g, crow, tile, wbase,
-                                                                         phase);
+            return strided_tma_tile_w<T, FUSE_PRE, BULK, DIR, kNarrowLinesF64>(map, map_out, a, g, crow, tile, wbase,
+                                                                              phase);
     }
-    return strided_tma_tile_w<T, FUSE_PRE, BULK, 32>(map, map_out, a, g, crow, tile, wbase, phase);
+    return strided_tma_tile_w<T, FUSE_PRE, BULK, DIR, 32>(map, map_out, a, g, crow, tile, wbase, phase);
 }
 
 // One warp tile of the pipelined z sweep (rows row0 .. row0 + R - 1 of
 // `tile`) in the warp's region `wbase`; mbarriers and `phase` as for
-// strided_tma_tile. Returns false (error flag set) when a bounded wait ran out.
-template <typename T, int SC>
+// strided_tma_tile, DIR as for strided_solve. Returns false (error flag set)
+// when a bounded wait ran out.
+template <typename T, int SC, bool DIR = true>
 __device__ __forceinline__ bool contig_pipe_tile(const SweepArgs<T> &a, const ContigGeom &g, int kc, long long tile,
                                                  unsigned char *wbase, unsigned phase) {
     const int lane = threadIdx.x & 31;
@@ -222,11 +241,15 @@ __device__ __forceinline__ bool contig_pipe_tile(const SweepArgs<T> &a, const Co
     const int d = active ? lane - r * S : 0;
     const long long row = row0 + r;
     const int i = (int)(row / a.ny), j = (int)(row % a.ny);
-    const unsigned m = (a.dir.any && active) ? a.dir.mask[d] : 0u;
+    const unsigned m = (DIR && a.dir.any && active) ? a.dir.mask[d] : 0u;
     const bool line_dir = ((m & 1u) && i == 0) || ((m & 2u) && i == a.nx - 1) || ((m & 4u) && j == 0) ||
                           ((m & 8u) && j == a.ny - 1);
     const bool lo_dir = m & 16u, hi_dir = m & 32u;
     T *line = sm + (size_t)r * g.RS + d;
+    // the end rows' face values, read while the tile's copies are in flight
+    const T g_lo = lo_dir ? dir_value(a.dir, i, j, 0, d) : T(0);
+    const T g_hi = hi_dir ? dir_value(a.dir, i, j, nz - 1, d) : T(0);
+    const bool solve = active && !line_dir;  // a line wholly on a face of another axis takes the face's values
     LineSolver<T> Ls(a, d);
     const int m0 = a.fac.m0;
 
@@ -235,40 +258,43 @@ __device__ __forceinline__ bool contig_pipe_tile(const SweepArgs<T> &a, const Co
     const int ref_c = kref / kc;
     for (int c = 0; c <= ref_c; ++c)
         if (!wait_c(c)) return false;
-    if (active) line[0] = Ls.first(line[0], line[kref * S]);
+    if (solve) line[0] = Ls.first(line[0], line[kref * S]);
     int k = 1;
     for (int c = 0; c < nch; ++c) {
         if (c > ref_c && !wait_c(c)) return false;
+        if (line_dir)
+            face_run_copy(face_run(a.dir, 2, i, j, 0, d), line, S, c * kc, min(nz, (c + 1) * kc));
         const int kend = min(nz - 1, (c + 1) * kc);
-        if (active) {
+        if (solve) {
             const int hend = min(kend, m0);
             k = head_forward(Ls, k, hend, [&](int q) { return line[q * S]; }, [&](int q, T v) { line[q * S] = v; });
             k = tail_forward(Ls, k, kend, [&](int q) { return line[q * S]; }, [&](int q, T v) { line[q * S] = v; });
         }
         k = max(k, kend);
     }
-    if (active && nz > 1) Ls.template fwd<false>(line[(nz - 1) * S], nz - 1);
+    if (solve && nz > 1) Ls.template fwd<false>(line[(nz - 1) * S], nz - 1);
 
     // ---- backward; each finished row group is stored for all rows of the tile
-    if (active) {
-        const T y = Ls.out_last();  // also seeds the back substitution
-        line[(nz - 1) * S] = (hi_dir || (lo_dir && nz == 1)) ? dir_value(a.dir, i, j, nz - 1, d) : y;
+    if (solve) {
+        T y = Ls.out_last();  // also seeds the back substitution
+        if (lo_dir && nz == 1) y = g_lo;
+        if (hi_dir) y = g_hi;
+        line[(nz - 1) * S] = y;
     }
     const int tl = max(m0, 1);
     k = nz - 2;
     for (int c = nch - 1; c >= 0; --c) {
         const int klo = c * kc;
-        if (active) {
+        if (line_dir) cp_wait<0>();  // the face values have landed
+        if (solve) {
             const int tstop = max(klo, tl);
             k = tail_backward(Ls, k, tstop, [&](int q) { return line[q * S]; }, [&](int q, T v) { line[q * S] = v; });
             const int hstop = max(klo, 1);
             k = head_backward(Ls, k, hstop, [&](int q) { return line[q * S]; }, [&](int q, T v) { line[q * S] = v; });
             if (klo == 0 && nz > 1) {
                 const T y = Ls.template bwd<false>(line[0], 0);
-                line[0] = lo_dir ? dir_value(a.dir, i, j, 0, d) : y;
+                line[0] = lo_dir ? g_lo : y;
             }
-            if (line_dir)
-                for (int q = klo; q < min(nz, klo + kc); ++q) line[q * S] = dir_value(a.dir, i, j, q, d);
         }
         k = min(k, klo - 1);
         fence_async_smem();

@@ -154,6 +154,31 @@ def test_random_shapes_fp64_bitexact(bfb, oracle, rng, shape, S, tma):
     assert np.array_equal(env.get_field(), want)
 
 
+@pytest.mark.parametrize("face", range(6))
+@pytest.mark.parametrize("shape,S", [((2, 3, 4), 1), ((3, 47, 5), 3), ((25, 24, 26), 2), ((49, 50, 17), 5),
+                                     ((1, 33, 48), 8), ((97, 6, 71), 1)])
+def test_lines_on_one_face_bitexact(bfb, oracle, rng, shape, S, face):
+    """One active face with a value per voxel, every substrate but the second: its lines hold
+    the face's values in the two sweeps along it, beside solved lines of the same tile, with
+    row groups and 24-row blocks ending anywhere; FP64 and FP32 bit for bit."""
+    D, lam = log_uniform(rng, 1e2, 1e5, S), log_uniform(rng, 1e-3, 1.0, S)
+    rho0 = rng.random((*shape, S))
+    vals = rng.random((*shape, S)) * 30
+    act = np.ones(S, np.uint8)
+    act[1:2] = 0
+    fm = np.zeros((6, S), np.uint8)
+    fm[face] = 1
+    mask = fm * act[None, :]
+    for prec in (bfb.FP64, bfb.FP32):
+        env = make_env(bfb, rho0, D, lam, prec)
+        env.set_dirichlet(act, values=vals, face_mask=fm)
+        env.diffusion_step(0.01, 2)
+        if prec == bfb.FP64:
+            assert np.array_equal(env.get_field(), oracle.lod_steps(rho0, 0.01, 20.0, D, lam, 2, vals, mask))
+        else:
+            assert np.array_equal(env.get_field_raw(), oracle.lod_steps_f32(rho0, 0.01, 20.0, D, lam, 2, vals, mask))
+
+
 @pytest.mark.parametrize("tma", [1, 0], ids=["tma", "cpasync"])
 @pytest.mark.parametrize("shape,S", SHAPES)
 def test_random_shapes_fp32(bfb, oracle, rng, shape, S, tma):
