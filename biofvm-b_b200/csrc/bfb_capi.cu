@@ -10,6 +10,7 @@
 
 #include "bfb_aux.cuh"
 #include "bfb_internal.cuh"
+#include "bfb_recip.h"
 #include "bfb_sweeps.cuh"
 
 namespace bfb {
@@ -111,7 +112,10 @@ static int tail_start(const std::vector<std::vector<double>> &tabs, int n, int S
 }
 
 // The device tables for one axis from the reference's factors (den, c).
-//   FP64: den and c as they are, and RN(1/den) for the division (div_rcp).
+//   FP64: den and c as they are, and RN(1/den) for the division (div_rcp),
+//         with the low term of the two-term reciprocal (div_rcp2) for the
+//         rows up to the constant tail; Factors::fast says where all of them
+//         are proven.
 //   FP32: 1/den as a hi+lo pair of floats, c1/den and c rounded once; the
 //         deviation form of the FP32 kernels (bfb_sweeps.cuh) needs no c1.
 static int upload_factors(bfb_env_s *env, int axis, int n, const std::vector<double> &den,
@@ -137,6 +141,17 @@ static int upload_factors(bfb_env_s *env, int axis, int n, const std::vector<dou
         tabs = {rh, rl, a, cf};
     }
     const int m0 = tail_start(tabs, n, S);
+    int fast = 0;
+    if (env->precision == BFB_FP64) {
+        std::vector<double> rl(nS, 0.0);
+        fast = kFastTail | kFastHead;
+        for (int m = 1; m <= std::min(m0, n - 1); ++m)
+            for (int d = 0; d < S; ++d) {
+                const size_t q = (size_t)m * S + d;
+                if (!two_term_reciprocal(den[q], tabs[2][q], &rl[q])) fast &= ~(m < m0 ? kFastHead : kFastTail);
+            }
+        tabs.push_back(rl);
+    }
     std::vector<double> flat, tail(4 * (size_t)S, 0.0);
     flat.reserve(4 * nS);
     for (size_t k = 0; k < 4; ++k) {
@@ -161,6 +176,7 @@ static int upload_factors(bfb_env_s *env, int axis, int n, const std::vector<dou
     st = upload_table(env, env->fac_head[axis], head);
     if (st) return st;
     env->fac_m0[axis] = m0;
+    env->fac_fast[axis] = fast;
     env->fac_hpad[axis] = hpad;
     return BFB_OK;
 }
@@ -215,6 +231,7 @@ static SweepArgs<T> make_args(bfb_env_s *env, int axis, bool bulk, double dt) {
     a.fac.head = static_cast<const T *>(env->fac_head[axis]);
     a.fac.m0 = env->fac_m0[axis];
     a.fac.hpad = env->fac_hpad[axis];
+    a.fac.fast = env->fac_fast[axis];
     a.c1 = static_cast<const T *>(env->c1);
     a.g = static_cast<const T *>(env->g);
     for (int f = 0; f < 6; ++f) a.dir.face[f] = static_cast<const T *>(env->faces[f]);

@@ -116,13 +116,14 @@ struct bfb_env_s {
     bool factors_valid = false;
     double factor_dt = 0;
     int freeze_factors = 1;
-    // per axis: tables [4][n*S] (FP64 uses 2: den, c; FP32 uses 4: 1/den hi,
+    // per axis: tables [4][n*S] (FP64: den, c, 1/den hi, lo; FP32: 1/den hi,
     // 1/den lo, c1/den, c) and tail values [4][S] for rows [m0, n-2]
     void *fac_tab[3] = {nullptr, nullptr, nullptr};
     void *fac_tail[3] = {nullptr, nullptr, nullptr};
     void *fac_head[3] = {nullptr, nullptr, nullptr};
     int fac_hpad[3] = {4, 4, 4};
     int fac_m0[3] = {1, 1, 1};
+    int fac_fast[3] = {0, 0, 0};         // Factors::fast
     void *c1 = nullptr;                  // [S] (FP64)
     void *g = nullptr;                   // [2*S] (FP32): 1/(1 + c2) as hi, lo
 

@@ -54,7 +54,8 @@ namespace bfb {
 constexpr int kChunks = 4;  // default row groups per tile (async copy / TMA stages)
 
 // Per-axis factor tables on the device (see bfb_capi.cu: upload_factors).
-//   FP64: t0 = den, t1 = c (back-substitution coefficient), t2 = RN(1/den)
+//   FP64: t0 = den, t1 = c (back-substitution coefficient), t2 = RN(1/den),
+//         t3 = the low term of the two-term reciprocal (bfb_recip.h)
 //   FP32: t0 = 1/den (hi), t1 = 1/den (lo), t2 = c1/den, t3 = c
 // tail[q*S + d] = value of table q on rows [m0, n-2] (valid when m0 <= n-2).
 // head[(q*S + d)*hpad + m] = table q, substrate d, row m < hpad: the rows
@@ -66,7 +67,9 @@ struct Factors {
     const T *tail;
     const T *head;
     int m0, hpad;
+    int fast;  // FP64: kFastTail / kFastHead where every divisor of those rows has a proven two-term reciprocal
 };
+constexpr int kFastTail = 1, kFastHead = 2;
 
 template <typename T>
 struct SweepArgs {
