@@ -139,15 +139,17 @@ __global__ void cells_kernel(T *__restrict__ f, int S, int nz, int Lp, int n_occ
     if (e >= (long long)n_occ * S) return;
     const int s = (int)(e / S), d = (int)(e % S);
     const size_t fe = voxel_elem(seg_voxel[s], d, nz, S, Lp);
+    const int a0 = seg_start[s], a1 = seg_start[s + 1];
+    pdl_wait();  // the segments are host-made; the field is the sweep's
     T x = f[fe];
-    const int a1 = seg_start[s + 1];
-    for (int a = seg_start[s]; a < a1; ++a) {
+    for (int a = a0; a < a1; ++a) {
         const size_t q = (size_t)a * S + d;
         if constexpr (sizeof(T) == 8)
             x = __ddiv_rn(__dadd_rn(x, t1[q]), t2[q]);
         else
             x = __fdiv_rn(__fadd_rn(x, t1[q]), t2[q]);
     }
+    pdl_launch_dependents();
     f[fe] = x;
 }
 
@@ -309,14 +311,13 @@ int launch_cells(bfb_env_s *env, cudaStream_t s) {
     const long long tot = (long long)env->n_occ * env->S;
     const unsigned gb = (unsigned)((tot + 255) / 256);
     if (env->precision == BFB_FP64)
-        cells_kernel<double><<<gb, 256, 0, s>>>((double *)env->field, env->S, env->nz, env->Lp, env->n_occ,
-                                                env->seg_start,
-                                                env->seg_voxel, (const double *)env->ag_t1, (const double *)env->ag_t2);
+        BFB_CUDA(launch_pdl(cells_kernel<double>, gb, 256, 0, s, (double *)env->field, env->S, env->nz, env->Lp,
+                            env->n_occ, env->seg_start, env->seg_voxel, (const double *)env->ag_t1,
+                            (const double *)env->ag_t2));
     else
-        cells_kernel<float><<<gb, 256, 0, s>>>((float *)env->field, env->S, env->nz, env->Lp, env->n_occ,
-                                               env->seg_start,
-                                               env->seg_voxel, (const float *)env->ag_t1, (const float *)env->ag_t2);
-    BFB_CUDA(cudaGetLastError());
+        BFB_CUDA(launch_pdl(cells_kernel<float>, gb, 256, 0, s, (float *)env->field, env->S, env->nz, env->Lp,
+                            env->n_occ, env->seg_start, env->seg_voxel, (const float *)env->ag_t1,
+                            (const float *)env->ag_t2));
     return BFB_OK;
 }
 

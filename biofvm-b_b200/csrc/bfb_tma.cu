@@ -48,6 +48,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 : 1)
         fence_mbar_init();
     }
     __syncwarp();
+    pdl_wait();
     strided_tma_tile<T, FUSE_PRE, BULK, DIR>(&map, &map_out, a, g, crow, tile, wbase, 0u);
 }
 
@@ -160,6 +161,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 : 1)
         fence_mbar_init();
     }
     __syncwarp();
+    pdl_wait();
     contig_pipe_tile<T, SC, DIR>(a, g, kc, tile, wbase, 0u);
 }
 
@@ -203,15 +205,11 @@ int launch_strided_tma(const SweepArgs<T> &a, const StridedGeom &g_in, const CUt
     const long long tiles = (long long)g.n_slabs * g.ncb;
     const unsigned blocks = (unsigned)((tiles + warps - 1) / warps);
     const size_t smem = wb * warps;
-    if (fuse_pre && a.bulk.on)
-        sweep_strided_tma_kernel<T, true, true, true><<<blocks, warps * 32, smem, s>>>(*map, *map_out, a, g, crow);
-    else if (fuse_pre && a.dir.any)
-        sweep_strided_tma_kernel<T, true, false, true><<<blocks, warps * 32, smem, s>>>(*map, *map_out, a, g, crow);
-    else if (a.dir.any)
-        sweep_strided_tma_kernel<T, false, false, true><<<blocks, warps * 32, smem, s>>>(*map, *map_out, a, g, crow);
-    else
-        sweep_strided_tma_kernel<T, false, false, false><<<blocks, warps * 32, smem, s>>>(*map, *map_out, a, g, crow);
-    BFB_CUDA(cudaGetLastError());
+    const auto kernel = fuse_pre && a.bulk.on     ? sweep_strided_tma_kernel<T, true, true, true>
+                        : fuse_pre && a.dir.any ? sweep_strided_tma_kernel<T, true, false, true>
+                        : a.dir.any             ? sweep_strided_tma_kernel<T, false, false, true>
+                                                : sweep_strided_tma_kernel<T, false, false, false>;
+    BFB_CUDA(launch_pdl(kernel, blocks, warps * 32, smem, s, *map, *map_out, a, g, crow));
     return BFB_OK;
 }
 
@@ -230,11 +228,9 @@ int launch_contig_tma(const SweepArgs<T> &a, const ContigGeom &g, int warps, cud
         for (int v = a.S * eb; v % 2 == 0 && q > 1; v /= 2) q /= 2;  // q = 16 / gcd(16, S*elem)
         int kc = (g.nz + chunks - 1) / chunks;
         kc = (kc + q - 1) / q * q;
-#define BFB_PIPE(SC)                                                                                  \
-    do {                                                                                              \
-        if (a.dir.any) sweep_contig_pipe_kernel<T, SC, true><<<blocks, warps * 32, smem, s>>>(a, g, kc); \
-        else sweep_contig_pipe_kernel<T, SC, false><<<blocks, warps * 32, smem, s>>>(a, g, kc);       \
-    } while (0)
+#define BFB_PIPE(SC)                                                                                             \
+    BFB_CUDA(launch_pdl(a.dir.any ? sweep_contig_pipe_kernel<T, SC, true> : sweep_contig_pipe_kernel<T, SC, false>, \
+                        blocks, warps * 32, smem, s, a, g, kc))
         switch (a.S) {
         case 1: BFB_PIPE(1); break;
         case 2: BFB_PIPE(2); break;

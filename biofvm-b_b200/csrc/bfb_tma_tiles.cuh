@@ -180,6 +180,7 @@ __device__ __forceinline__ bool strided_tma_tile_w(const CUtensorMap *map, const
         }
     };
     if (!strided_solve<T, FUSE_PRE, BULK, DIR, TW>(a, g, crow, slab, col0, sm + lane, wait, flush)) return false;
+    pdl_launch_dependents();
     if (lane == 0) bulk_wait_read_all();  // the tile must outlive the stores' reads
     __syncwarp();
     return true;
@@ -306,6 +307,7 @@ __device__ __forceinline__ bool contig_pipe_tile(const SweepArgs<T> &a, const Co
             bulk_commit();
         }
     }
+    pdl_launch_dependents();
     if (lane == 0) bulk_wait_read_all();
     __syncwarp();
     return true;

@@ -222,6 +222,43 @@ def test_factors_without_a_constant_tail(bfb, oracle, rng):
     assert np.array_equal(env.get_field(), oracle.lod_steps(rho0, 0.01, 20.0, D, lam, 2))
 
 
+@pytest.mark.parametrize("calls", [(1,) * 12, (8, 8, 8, 8, 9, 1), (40, 3, 17), (7, 31, 16, 5)])
+def test_simulate_launches_and_graph_agree(bfb, oracle, rng, calls):
+    """bfb_simulate issues steps as launches, then as graphs of eight steps and a remainder of
+    launches; the fields equal the oracle's after every call, also when the Dirichlet values and
+    the flags change between calls."""
+    shape, S = (13, 9, 11), 2
+    D, lam = log_uniform(rng, 1e2, 1e5, S), log_uniform(rng, 1e-3, 1.0, S)
+    want = rng.random((*shape, S))
+    n = 60
+    pos = rng.random((n, 3)) * np.array(shape) * 20.0
+    vol = np.full(n, 500.0)
+    sec, upt, sat = log_uniform(rng, 1e-2, 10.0, (3, n, S))
+    env = make_env(bfb, want, D, lam, bfb.FP64)
+    env.set_agents(pos, vol, sec, upt, sat, 0.01)
+    vox = oracle.bin_agents(pos, (0.0, 0.0, 0.0, *(20.0 * v for v in shape)), 20.0, shape)
+    t1, t2 = oracle.agent_constants(0.01, 20.0, vol, sec, upt, sat)
+    for q, steps in enumerate(calls):
+        vals = None
+        if q % 3 == 2:
+            vals = rng.random((*shape, S))
+            env.set_dirichlet(np.ones(S, np.uint8), values=vals)
+        elif q % 3 == 0:
+            env.set_dirichlet(np.zeros(S, np.uint8))
+        if q % 3 != 1:
+            last = vals
+        cells = q % 2 == 0
+        env.simulate(0.01, steps, bfb.STEP_DIFFUSION | (bfb.STEP_CELLS if cells else 0))
+        for _ in range(steps):
+            if last is None:
+                want = oracle.lod_steps(want, 0.01, 20.0, D, lam, 1)
+            else:
+                want = oracle.lod_steps(want, 0.01, 20.0, D, lam, 1, last, face_mask_all(np.ones(S)))
+            if cells:
+                want = oracle.cells_step(want, vox, t1, t2)
+        assert np.array_equal(env.get_field(), want)
+
+
 def test_agents_random_fp64_and_fp32(bfb, oracle, rng):
     shape, S = (20, 18, 16), 3
     dx, dt = 20.0, 0.01
