@@ -216,9 +216,9 @@ __global__ void __launch_bounds__(128, (TMA_ONLY && sizeof(T) == 4) ? 4 : 1) bat
                 if (stage < 2 && I.tma[stage]) {
                     const StridedGeom &g = stage == 0 ? I.gx : I.gy;
                     const int crow = I.crow[stage];
-                    ok = stage == 0 ? strided_tma_tile<T, true, false>(I.map[0], I.map[0], I.ax[0], g, crow, tile,
+                    ok = stage == 0 ? strided_tma_tile<T, true>(I.map[0], I.map[0], I.ax[0], g, crow, tile,
                                                                        wbase, phase)
-                                    : strided_tma_tile<T, false, false>(I.map[1], I.map[1], I.ax[1], g, crow, tile,
+                                    : strided_tma_tile<T, false>(I.map[1], I.map[1], I.ax[1], g, crow, tile,
                                                                         wbase, phase);
                     phase ^= (1u << ((g.n + crow - 1) / crow)) - 1u;
                     groups += (g.n + crow - 1) / crow;  // one store group per row group
@@ -234,11 +234,11 @@ __global__ void __launch_bounds__(128, (TMA_ONLY && sizeof(T) == 4) ? 4 : 1) bat
                     groups += (I.gz.nz + I.kc - 1) / I.kc;
                 } else if constexpr (!TMA_ONLY) {
                     if (stage == 0) {
-                        if (I.vb16[0]) strided_tile<T, 16, true, false>(I.ax[0], I.gx, tile, sm);
-                        else strided_tile<T, (int)sizeof(T), true, false>(I.ax[0], I.gx, tile, sm);
+                        if (I.vb16[0]) strided_tile<T, 16, true>(I.ax[0], I.gx, tile, sm);
+                        else strided_tile<T, (int)sizeof(T), true>(I.ax[0], I.gx, tile, sm);
                     } else if (stage == 1) {
-                        if (I.vb16[1]) strided_tile<T, 16, false, false>(I.ax[1], I.gy, tile, sm);
-                        else strided_tile<T, (int)sizeof(T), false, false>(I.ax[1], I.gy, tile, sm);
+                        if (I.vb16[1]) strided_tile<T, 16, false>(I.ax[1], I.gy, tile, sm);
+                        else strided_tile<T, (int)sizeof(T), false>(I.ax[1], I.gy, tile, sm);
                     } else {
                         if (I.vb16[2]) contig_tile_any<T, 16>(I.ax[2], I.gz, tile, sm);
                         else contig_tile_any<T, (int)sizeof(T)>(I.ax[2], I.gz, tile, sm);
@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(128, (sizeof(T) == 4 && PATH == kPathTma && ST
             if constexpr (STAGE < 2) {
                 const StridedGeom g = STAGE == 0 ? I.gx : I.gy;
                 const CUtensorMap *mp = I.map[STAGE];
-                strided_tma_tile<T, STAGE == 0, false>(mp, mp, ax, g, I.crow[STAGE], tile, wbase, 0u);
+                strided_tma_tile<T, STAGE == 0>(mp, mp, ax, g, I.crow[STAGE], tile, wbase, 0u);
             } else {
                 const ContigGeom gz = I.gz;
                 switch (I.S) {  // the substrate count as a constant where it is a common one
@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(128, (sizeof(T) == 4 && PATH == kPathTma && ST
             constexpr int VB = PATH == kPathCp16 ? 16 : (int)sizeof(T);
             if constexpr (STAGE < 2) {
                 const StridedGeom g = STAGE == 0 ? I.gx : I.gy;
-                strided_tile<T, VB, STAGE == 0, false>(ax, g, tile, sm);
+                strided_tile<T, VB, STAGE == 0>(ax, g, tile, sm);
             } else {
                 contig_tile_any<T, VB>(ax, I.gz, tile, sm);
             }

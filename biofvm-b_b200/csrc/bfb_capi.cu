@@ -267,15 +267,13 @@ static void encode_field_maps(bfb_env_s *env) {
     }
 }
 
-// One LOD diffusion step; `bulk` fuses a preceding bulk source/sink update
-// into the x-sweep load.
 template <typename T>
-static int launch_strided_env(bfb_env_s *env, int axis, bool bulk, double dt, cudaStream_t s) {
-    const SweepArgs<T> a = make_args<T>(env, axis, bulk, dt);
+static int launch_strided_env(bfb_env_s *env, int axis, double dt, cudaStream_t s) {
+    const SweepArgs<T> a = make_args<T>(env, axis, false, dt);
     if constexpr (sizeof(T) == 8) {  // the tensor-memory tiles where the tuning asks for them
         if (env->use_tma && env->tuning.tma[axis] == 2 && env->tmem_ok[axis]) {
             const int st = launch_strided_tmem(a, strided_geometry(a, axis), &env->tmem_map[axis],
-                                               &env->tmem_map[axis], axis == 0 && (a.dir.any || a.bulk.on), s);
+                                               &env->tmem_map[axis], axis == 0 && a.dir.any, s);
             if (st != kNotApplicable) return st;
         }
     }
@@ -290,11 +288,11 @@ static int refuse_slab(const bfb_env_s *env) {
 }
 
 template <typename T>
-static int run_diffusion(bfb_env_s *env, double dt, bool bulk, cudaStream_t s) {
+static int run_diffusion(bfb_env_s *env, double dt, cudaStream_t s) {
     if (int st = refuse_slab(env)) return st;
-    int st = launch_strided_env<T>(env, 0, bulk, dt, s);
+    int st = launch_strided_env<T>(env, 0, dt, s);
     if (st) return st;
-    st = launch_strided_env<T>(env, 1, false, dt, s);
+    st = launch_strided_env<T>(env, 1, dt, s);
     if (st) return st;
     return launch_contig<T>(make_args<T>(env, 2, false, dt), env->tuning.warps[2],
                             env->use_tma != 0 && env->tuning.tma[2] != 0, s, env->tuning.chunks[2]);
@@ -304,11 +302,8 @@ template <typename T>
 static int run_steps(bfb_env_s *env, double dt, int n, int flags, cudaStream_t s) {
     for (int q = 0; q < n; ++q) {
         int st = BFB_OK;
-        if (flags & BFB_STEP_DIFFUSION) {
-            st = run_diffusion<T>(env, dt, (flags & BFB_STEP_BULK) != 0, s);
-        } else if (flags & BFB_STEP_BULK) {
-            st = launch_bulk<T>(make_args<T>(env, 0, true, dt), env->Np, s);
-        }
+        if (flags & BFB_STEP_BULK) st = launch_bulk<T>(make_args<T>(env, 0, true, dt), env->Np, s);
+        if (!st && (flags & BFB_STEP_DIFFUSION)) st = run_diffusion<T>(env, dt, s);
         if (st) return st;
         if (flags & BFB_STEP_CELLS) {
             st = launch_cells(env, s);
@@ -1190,16 +1185,18 @@ BFB_API int bfb_profile_steps(bfb_env env, double dt, int n_steps, int flags, do
     };
     for (int q = 0; q < n_steps && !st; ++q) {
         const bool fp64 = env->precision == BFB_FP64;
-        if (flags & BFB_STEP_DIFFUSION) {
-            const bool bulk = (flags & BFB_STEP_BULK) != 0;
+        if (flags & BFB_STEP_BULK)
+            st = phase_ms(3, [&] {
+                return fp64 ? launch_bulk<double>(make_args<double>(env, 0, true, dt), env->Np, s)
+                            : launch_bulk<float>(make_args<float>(env, 0, true, dt), env->Np, s);
+            });
+        if (!st && (flags & BFB_STEP_DIFFUSION)) {
             st = phase_ms(0, [&] {
-                return fp64 ? launch_strided_env<double>(env, 0, bulk, dt, s)
-                            : launch_strided_env<float>(env, 0, bulk, dt, s);
+                return fp64 ? launch_strided_env<double>(env, 0, dt, s) : launch_strided_env<float>(env, 0, dt, s);
             });
             if (!st)
                 st = phase_ms(1, [&] {
-                    return fp64 ? launch_strided_env<double>(env, 1, false, dt, s)
-                                : launch_strided_env<float>(env, 1, false, dt, s);
+                    return fp64 ? launch_strided_env<double>(env, 1, dt, s) : launch_strided_env<float>(env, 1, dt, s);
                 });
             if (!st)
                 st = phase_ms(2, [&] {
@@ -1209,11 +1206,6 @@ BFB_API int bfb_profile_steps(bfb_env env, double dt, int n_steps, int flags, do
                                 : launch_contig<float>(make_args<float>(env, 2, false, dt), env->tuning.warps[2], tz, s,
                                                        env->tuning.chunks[2]);
                 });
-        } else if (flags & BFB_STEP_BULK) {
-            st = phase_ms(3, [&] {
-                return fp64 ? launch_bulk<double>(make_args<double>(env, 0, true, dt), env->Np, s)
-                            : launch_bulk<float>(make_args<float>(env, 0, true, dt), env->Np, s);
-            });
         }
         if (!st && (flags & BFB_STEP_CELLS)) st = phase_ms(4, [&] { return launch_cells(env, s); });
     }
@@ -1314,7 +1306,7 @@ BFB_API int bfb_slab_yz(bfb_env env, double dt) {
     if (st) return st;
     if ((st = slab_half_args(env, dt, 0, 0))) return st;
     NvtxRange range("bfb_slab_yz");
-    if ((st = launch_strided_env<double>(env, 1, false, dt, env->stream))) return st;
+    if ((st = launch_strided_env<double>(env, 1, dt, env->stream))) return st;
     return launch_contig<double>(make_args<double>(env, 2, false, dt), env->tuning.warps[2],
                                  env->use_tma != 0 && env->tuning.tma[2] != 0, env->stream, env->tuning.chunks[2]);
 }

@@ -96,7 +96,7 @@ struct DirFaces {
     int any;              // 0: no active face for any substrate
 };
 
-// Bulk source/sink terms fused into the x-sweep load.
+// Bulk source/sink terms, applied before the x sweep (bulk_kernel).
 //   A = S*T (rounded once), B = U + S (rounded once); rho <- (rho + dt*A) / (B*dt + 1)
 template <typename T>
 struct BulkTerms {

@@ -20,9 +20,9 @@
 //     contiguous elements. A warp stages R = 32/S whole rows (one contiguous
 //     block of global memory) into padded shared rows, lane (r, d) solves line
 //     (row r, substrate d) in place, and the warp copies the rows back out.
-// Dirichlet is fused: the pre-X Dir (and, if enabled, the bulk source/sink
-// update that precedes the step) on the X-sweep load, and each post-sweep Dir
-// on that sweep's store. Because Dir is a pure overwrite of fixed positions
+// Dirichlet is fused: the pre-X Dir on the X-sweep load, and each post-sweep Dir
+// on that sweep's store. (The bulk source/sink update that may precede the step
+// is a launch of its own, see bulk_kernel.) Because Dir is a pure overwrite of fixed positions
 // and each sweep rewrites every element of its line, this is exactly the
 // reference's sequence. The recurrence keeps the un-overwritten values.
 //
@@ -109,7 +109,7 @@ struct ContigGeom {
 // The voxel and substrate of strided column `cl` of slab `slab` (x: cl =
 // j*Lp + q, y: cl = q, with q = k*S + d); `real` is false for columns past P
 // and for the padding of a padded row (q >= nz*S), whose lanes run along but
-// read no Dirichlet value or bulk term.
+// read no Dirichlet value.
 struct StridedColumn {
     int d, ci, cj, ck;
     bool real;

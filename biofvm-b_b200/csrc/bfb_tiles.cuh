@@ -9,7 +9,7 @@ namespace bfb {
 // One strided tile (32 lines of one slab) by the calling warp; sm is the
 // warp's shared-memory region of n*32 elements. Used by the single-env kernel
 // below and by the batched ensemble kernel (bfb_batch.cu).
-template <typename T, int VB, bool FUSE_PRE, bool BULK>
+template <typename T, int VB, bool FUSE_PRE>
 __device__ __forceinline__ void strided_tile(const SweepArgs<T> &a, const StridedGeom &g, long long tile, T *sm) {
     const int lane = threadIdx.x & 31;
     const int slab = (int)(tile / g.ncb);
@@ -58,7 +58,7 @@ __device__ __forceinline__ void strided_tile(const SweepArgs<T> &a, const Stride
     }
 
     // ---- line coordinates of this lane (padding columns of a padded row run
-    // along with no Dirichlet value and no bulk term)
+    // along with no Dirichlet value)
     const long long col = col0 + lane;
     const StridedColumn col_at = strided_column(a, g, slab, col);
     const int d = col_at.d, ci = col_at.ci, cj = col_at.cj, ck = col_at.ck;
@@ -78,18 +78,7 @@ __device__ __forceinline__ void strided_tile(const SweepArgs<T> &a, const Stride
     auto vox_dir = [&](int mm) -> T {
         return g.axis == 0 ? dir_value(a.dir, mm, cj, ck, d) : dir_value(a.dir, ci, mm, ck, d);
     };
-    const T *bA = nullptr, *bB = nullptr;
-    if constexpr (BULK) {
-        bA = a.bulk.A + (size_t)slab * g.slab_stride + col;
-        bB = a.bulk.B + (size_t)slab * g.slab_stride + col;
-    }
-    auto load = [&](int r) -> T {
-        T x = sm[r * 32 + lane];
-        if constexpr (BULK) {
-            if (col_at.real) x = bulk_update(x, bA[(size_t)r * P], bB[(size_t)r * P], a.bulk.dt);
-        }
-        return x;
-    };
+    auto load = [&](int r) -> T { return sm[r * 32 + lane]; };
 
     LineSolver<T> L(a, d);
     const int m0 = a.fac.m0;

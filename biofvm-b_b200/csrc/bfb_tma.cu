@@ -32,7 +32,7 @@ namespace bfb {
 // per SM instead of 17. Large grids are bound by shared memory and do not
 // change; many small envs stepped side by side do (256 grids of edges 32-160
 // stepped one env at a time: 6.70 -> 6.35 ms per step).
-template <typename T, bool FUSE_PRE, bool BULK, bool DIR>
+template <typename T, bool FUSE_PRE, bool DIR>
 __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 : 1)
     sweep_strided_tma_kernel(const __grid_constant__ CUtensorMap map, const __grid_constant__ CUtensorMap map_out,
                              SweepArgs<T> a, StridedGeom g, int crow) {
@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 : 1)
     }
     __syncwarp();
     pdl_wait();
-    strided_tma_tile<T, FUSE_PRE, BULK, DIR>(&map, &map_out, a, g, crow, tile, wbase, 0u);
+    strided_tma_tile<T, FUSE_PRE, DIR>(&map, &map_out, a, g, crow, tile, wbase, 0u);
 }
 
 // ---------------------------------------------------------------------------
@@ -205,10 +205,9 @@ int launch_strided_tma(const SweepArgs<T> &a, const StridedGeom &g_in, const CUt
     const long long tiles = (long long)g.n_slabs * g.ncb;
     const unsigned blocks = (unsigned)((tiles + warps - 1) / warps);
     const size_t smem = wb * warps;
-    const auto kernel = fuse_pre && a.bulk.on     ? sweep_strided_tma_kernel<T, true, true, true>
-                        : fuse_pre && a.dir.any ? sweep_strided_tma_kernel<T, true, false, true>
-                        : a.dir.any             ? sweep_strided_tma_kernel<T, false, false, true>
-                                                : sweep_strided_tma_kernel<T, false, false, false>;
+    const auto kernel = fuse_pre && a.dir.any ? sweep_strided_tma_kernel<T, true, true>
+                        : a.dir.any           ? sweep_strided_tma_kernel<T, false, true>
+                                              : sweep_strided_tma_kernel<T, false, false>;
     BFB_CUDA(launch_pdl(kernel, blocks, warps * 32, smem, s, *map, *map_out, a, g, crow));
     return BFB_OK;
 }
@@ -271,10 +270,9 @@ static void opt_in_pipe() {
 
 template <typename T>
 static void opt_in_tma_all() {
-    opt_in_tma(sweep_strided_tma_kernel<T, true, true, true>);
-    opt_in_tma(sweep_strided_tma_kernel<T, true, false, true>);
-    opt_in_tma(sweep_strided_tma_kernel<T, false, false, true>);
-    opt_in_tma(sweep_strided_tma_kernel<T, false, false, false>);
+    opt_in_tma(sweep_strided_tma_kernel<T, true, true>);
+    opt_in_tma(sweep_strided_tma_kernel<T, false, true>);
+    opt_in_tma(sweep_strided_tma_kernel<T, false, false>);
     opt_in_pipe<T, 1>();
     opt_in_pipe<T, 2>();
     opt_in_pipe<T, 3>();
@@ -358,7 +356,7 @@ bool make_sweep_tensor_map_rows(CUtensorMap *out, void *field, int elem, int axi
 int strided_tile_lines(int n, int elem, int chunks) {
     if (elem != 8) return 32;
     if (chunks < 1) chunks = 1;
-    const void *kernel = (const void *)sweep_strided_tma_kernel<double, false, false, false>;
+    const void *kernel = (const void *)sweep_strided_tma_kernel<double, false, false>;
     auto resident = [&](int w) -> long long {  // lines per SM at width w (0: does not fit)
         const int crow = strided_box_rows(n, chunks, w, elem);
         const size_t wb = strided_tma_warp_bytes(n, crow, elem, w);

@@ -23,13 +23,12 @@ namespace bfb {
 // row by row instead, the tiles on a face took ten times the others' time and
 // were every sweep's tail (200^3 x 8 FP32, x faces of one substrate: y 194 ->
 // 101 us, z 169 -> 100 us; 75^3 x 1 FP64, all faces: step 78 -> 31 us).
-template <typename T, bool FUSE_PRE, bool BULK, bool DIR, int RS, typename WAIT, typename FLUSH>
+template <typename T, bool FUSE_PRE, bool DIR, int RS, typename WAIT, typename FLUSH>
 __device__ __forceinline__ bool strided_solve(const SweepArgs<T> &a, const StridedGeom &g, int crow, int slab,
                                               long long col0, T *__restrict__ col, WAIT wait, FLUSH flush) {
     constexpr int rs = RS;  // a compile-time row stride keeps the row loops free of address arithmetic
     const int lane = threadIdx.x & 31;
     const int n = g.n;
-    const long long P = g.P;
     const int nch = (n + crow - 1) / crow;
     if (lane >= rs) {  // no line: follow the row groups' waits and flushes
         for (int ch = 0; ch < nch; ++ch)
@@ -62,18 +61,7 @@ __device__ __forceinline__ bool strided_solve(const SweepArgs<T> &a, const Strid
     };
     // the end rows' face values, read while the tile's copies are in flight
     const T g_lo = lo_dir ? vox_dir(0) : T(0), g_hi = hi_dir ? vox_dir(n - 1) : T(0);
-    const T *bA = nullptr, *bB = nullptr;
-    if constexpr (BULK) {
-        bA = a.bulk.A + (size_t)slab * g.slab_stride + cl;
-        bB = a.bulk.B + (size_t)slab * g.slab_stride + cl;
-    }
-    auto load = [&](int r) -> T {
-        T x = col[r * rs];
-        if constexpr (BULK) {
-            if (valid) x = bulk_update(x, bA[(size_t)r * P], bB[(size_t)r * P], a.bulk.dt);
-        }
-        return x;
-    };
+    auto load = [&](int r) -> T { return col[r * rs]; };
 
     LineSolver<T> L(a, d);
     const int m0 = a.fac.m0;
@@ -146,7 +134,7 @@ __device__ __forceinline__ bool strided_solve(const SweepArgs<T> &a, const Strid
 // tile). The mbarriers are initialised by the caller; row group ch waits for
 // parity bit ch of `phase`, and every call completes one phase of each of
 // its row groups. Returns false (error flag set) when a bounded wait ran out.
-template <typename T, bool FUSE_PRE, bool BULK, bool DIR, int TW>
+template <typename T, bool FUSE_PRE, bool DIR, int TW>
 __device__ __forceinline__ bool strided_tma_tile_w(const CUtensorMap *map, const CUtensorMap *map_out,
                                                    const SweepArgs<T> &a, const StridedGeom &g, int crow,
                                                    long long tile, unsigned char *wbase, unsigned phase) {
@@ -179,7 +167,7 @@ __device__ __forceinline__ bool strided_tma_tile_w(const CUtensorMap *map, const
             bulk_commit();
         }
     };
-    if (!strided_solve<T, FUSE_PRE, BULK, DIR, TW>(a, g, crow, slab, col0, sm + lane, wait, flush)) return false;
+    if (!strided_solve<T, FUSE_PRE, DIR, TW>(a, g, crow, slab, col0, sm + lane, wait, flush)) return false;
     pdl_launch_dependents();
     if (lane == 0) bulk_wait_read_all();  // the tile must outlive the stores' reads
     __syncwarp();
@@ -187,16 +175,16 @@ __device__ __forceinline__ bool strided_tma_tile_w(const CUtensorMap *map, const
 }
 
 // The tile at the geometry's width: 32 lines, or kNarrowLinesF64 for FP64.
-template <typename T, bool FUSE_PRE, bool BULK, bool DIR = true>
+template <typename T, bool FUSE_PRE, bool DIR = true>
 __device__ __forceinline__ bool strided_tma_tile(const CUtensorMap *map, const CUtensorMap *map_out,
                                                  const SweepArgs<T> &a, const StridedGeom &g, int crow, long long tile,
                                                  unsigned char *wbase, unsigned phase) {
     if constexpr (sizeof(T) == 8) {
         if (g.tw == kNarrowLinesF64)
-            return strided_tma_tile_w<T, FUSE_PRE, BULK, DIR, kNarrowLinesF64>(map, map_out, a, g, crow, tile, wbase,
+            return strided_tma_tile_w<T, FUSE_PRE, DIR, kNarrowLinesF64>(map, map_out, a, g, crow, tile, wbase,
                                                                               phase);
     }
-    return strided_tma_tile_w<T, FUSE_PRE, BULK, DIR, 32>(map, map_out, a, g, crow, tile, wbase, phase);
+    return strided_tma_tile_w<T, FUSE_PRE, DIR, 32>(map, map_out, a, g, crow, tile, wbase, phase);
 }
 
 // One warp tile of the pipelined z sweep (rows row0 .. row0 + R - 1 of

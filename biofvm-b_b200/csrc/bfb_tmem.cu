@@ -120,12 +120,11 @@ __device__ __forceinline__ void bulk_wait_read_n() {
 
 // One warp's tiles (32 lines each): tile w, w + W, ... of the sweep. Returns
 // false when a bounded wait ran out (the error flag is set).
-template <bool FUSE_PRE, bool BULK>
+template <bool FUSE_PRE>
 __device__ bool tmem_warp_tiles(const CUtensorMap *map, const CUtensorMap *map_out, const SweepArgs<double> &a,
                                 const StridedGeom &g, unsigned char *wbase, unsigned tbase) {
     const int lane = threadIdx.x & 31;
     const int n = g.n;
-    const long long P = g.P;
     const int ng = (n + kTmemGroup - 1) / kTmemGroup;
     const long long ntiles = (long long)g.n_slabs * g.ncb;
     const long long stride = (long long)gridDim.x * kTmemWarps;
@@ -187,17 +186,6 @@ __device__ bool tmem_warp_tiles(const CUtensorMap *map, const CUtensorMap *map_o
         auto vox_dir = [&](int mm) -> double {
             return g.axis == 0 ? dir_value(a.dir, mm, cj, ck, d) : dir_value(a.dir, ci, mm, ck, d);
         };
-        const double *bA = nullptr, *bB = nullptr;
-        if constexpr (BULK) {
-            bA = a.bulk.A + (size_t)slab * g.slab_stride + cl;
-            bB = a.bulk.B + (size_t)slab * g.slab_stride + cl;
-        }
-        auto upd = [&](double x, int q) -> double {
-            if constexpr (BULK) {
-                if (valid) x = bulk_update(x, bA[(size_t)q * P], bB[(size_t)q * P], a.bulk.dt);
-            }
-            return x;
-        };
         LineSolver<double> L(a, d);
 
         // ---- forward elimination, group by group from the input ring, eight
@@ -219,7 +207,7 @@ __device__ bool tmem_warp_tiles(const CUtensorMap *map, const CUtensorMap *map_o
                 double y[8];
                 if (b >= tl && b + 8 <= n - 1) {  // tail rows only: factors in registers
 #pragma unroll
-                    for (int u = 0; u < 8; ++u) y[u] = upd(rows[u * 32], b + u);
+                    for (int u = 0; u < 8; ++u) y[u] = rows[u * 32];
 #pragma unroll
                     for (int u = 0; u < 8; ++u) y[u] = L.tstep(y[u]);
                 } else {
@@ -228,7 +216,7 @@ __device__ bool tmem_warp_tiles(const CUtensorMap *map, const CUtensorMap *map_o
                         const int q = b + u;
                         double v = 0.0;
                         if (q < n) {
-                            double x = upd(rows[u * 32], q);
+                            double x = rows[u * 32];
                             if (FUSE_PRE && ((q == 0 && lo_dir) || (q == n - 1 && hi_dir))) x = vox_dir(q);
                             if (q == 0)
                                 v = L.first(x, x);
@@ -326,7 +314,7 @@ __device__ bool tmem_warp_tiles(const CUtensorMap *map, const CUtensorMap *map_o
     return ok;
 }
 
-template <bool FUSE_PRE, bool BULK>
+template <bool FUSE_PRE>
 __global__ void __launch_bounds__(kTmemWarps * 32, 1)
     sweep_strided_tmem_kernel(const __grid_constant__ CUtensorMap map, const __grid_constant__ CUtensorMap map_out,
                               SweepArgs<double> a, StridedGeom g) {
@@ -342,7 +330,7 @@ __global__ void __launch_bounds__(kTmemWarps * 32, 1)
     tmem_fence_after_sync();
     const unsigned tmem = *taddr_slot;
     unsigned char *wbase = smem_raw + 128 + (size_t)warp * kTmemWarpBytes;
-    tmem_warp_tiles<FUSE_PRE, BULK>(&map, &map_out, a, g, wbase, tmem + ((unsigned)(warp * 32) << 16));
+    tmem_warp_tiles<FUSE_PRE>(&map, &map_out, a, g, wbase, tmem + ((unsigned)(warp * 32) << 16));
     tmem_fence_before_sync();
     __syncthreads();  // every warp is done with its TMEM lanes
     tmem_fence_after_sync();
@@ -370,9 +358,7 @@ bool make_tmem_sweep_map(CUtensorMap *out, void *field, int axis, int nx, int ny
 }
 
 void tmem_prepare_device() {
-    for (const void *k : {(const void *)sweep_strided_tmem_kernel<true, true>,
-                          (const void *)sweep_strided_tmem_kernel<true, false>,
-                          (const void *)sweep_strided_tmem_kernel<false, false>})
+    for (const void *k : {(const void *)sweep_strided_tmem_kernel<true>, (const void *)sweep_strided_tmem_kernel<false>})
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTmemCtaBytes);
 }
 
@@ -385,12 +371,10 @@ int launch_strided_tmem(const SweepArgs<double> &a, const StridedGeom &g_in, con
     const long long tiles = (long long)g.n_slabs * g.ncb;
     const long long blocks = std::min<long long>(sm_count(), (tiles + kTmemWarps - 1) / kTmemWarps);
     const unsigned grid = (unsigned)std::max<long long>(1, blocks);
-    if (fuse_pre && a.bulk.on)
-        sweep_strided_tmem_kernel<true, true><<<grid, kTmemWarps * 32, kTmemCtaBytes, s>>>(*map, *map_out, a, g);
-    else if (fuse_pre)
-        sweep_strided_tmem_kernel<true, false><<<grid, kTmemWarps * 32, kTmemCtaBytes, s>>>(*map, *map_out, a, g);
+    if (fuse_pre)
+        sweep_strided_tmem_kernel<true><<<grid, kTmemWarps * 32, kTmemCtaBytes, s>>>(*map, *map_out, a, g);
     else
-        sweep_strided_tmem_kernel<false, false><<<grid, kTmemWarps * 32, kTmemCtaBytes, s>>>(*map, *map_out, a, g);
+        sweep_strided_tmem_kernel<false><<<grid, kTmemWarps * 32, kTmemCtaBytes, s>>>(*map, *map_out, a, g);
     BFB_CUDA(cudaGetLastError());
     return BFB_OK;
 }

@@ -209,8 +209,8 @@ BFB_API int bfb_host_unregister(void *host);
  * CSV (BioFVM_parallel.cpp:695-697, 1259-1392): runs n_steps steps like
  * bfb_simulate (without a graph) with CUDA events around every launch and
  * adds the milliseconds of each phase to ms_out[BFB_PROFILE_PHASES]:
- * 0 x-sweep (with the fused pre-x Dirichlet / bulk), 1 y-sweep, 2 z-sweep,
- * 3 standalone bulk, 4 cells. */
+ * 0 x-sweep (with the fused pre-x Dirichlet), 1 y-sweep, 2 z-sweep, 3 bulk,
+ * 4 cells. */
 #define BFB_PROFILE_PHASES 5
 BFB_API int bfb_profile_steps(bfb_env env, double dt, int n_steps, int flags, double *ms_out);
 
