@@ -528,11 +528,11 @@ static int batch_upload(bfb_batch_s *b, double dt) {
             b->stage_base[s + 1][f] = b->stage_base[s][f] + cnt;
         }
     }
-    BFB_CUDA(cudaMemcpy(b->d_maps, maps.data(), sizeof(CUtensorMap) * maps.size(), cudaMemcpyHostToDevice));
-    BFB_CUDA(cudaMemcpy(b->d_inst, inst.data(), sizeof(BatchInst<T>) * b->n, cudaMemcpyHostToDevice));
-    BFB_CUDA(cudaMemcpy(b->d_prefix, prefix.data(), sizeof(int) * prefix.size(), cudaMemcpyHostToDevice));
-    BFB_CUDA(cudaMemcpy(b->d_tpre, tpre.data(), sizeof(int) * tpre.size(), cudaMemcpyHostToDevice));
-    BFB_CUDA(cudaMemcpy(b->d_perm, perm.data(), sizeof(int) * perm.size(), cudaMemcpyHostToDevice));
+    BFB_CUDA(cudaMemcpyAsync(b->d_maps, maps.data(), sizeof(CUtensorMap) * maps.size(), cudaMemcpyHostToDevice, b->stream));
+    BFB_CUDA(cudaMemcpyAsync(b->d_inst, inst.data(), sizeof(BatchInst<T>) * b->n, cudaMemcpyHostToDevice, b->stream));
+    BFB_CUDA(cudaMemcpyAsync(b->d_prefix, prefix.data(), sizeof(int) * prefix.size(), cudaMemcpyHostToDevice, b->stream));
+    BFB_CUDA(cudaMemcpyAsync(b->d_tpre, tpre.data(), sizeof(int) * tpre.size(), cudaMemcpyHostToDevice, b->stream));
+    BFB_CUDA(cudaMemcpyAsync(b->d_perm, perm.data(), sizeof(int) * perm.size(), cudaMemcpyHostToDevice, b->stream));
     b->tma_only = true;
     for (int k = 0; k < b->n; ++k) b->tma_only = b->tma_only && inst[k].tma[0] && inst[k].tma[1] && inst[k].tma[2];
     const void *step_kernel = b->tma_only ? (const void *)batch_step_kernel<T, true>
@@ -845,9 +845,10 @@ BFB_API int bfb_batch_autotune(bfb_batch b, double dt, int flags, int trials, in
     int st = BFB_OK;
     for (int k = 0; k < b->n && !st; ++k) {
         bfb_env_s *e = b->envs[k];
-        cudaError_t ce = cudaStreamSynchronize(e->stream);
-        if (ce == cudaSuccess) ce = cudaMalloc(&saved[k], e->elem * e->Np);
-        if (ce == cudaSuccess) ce = cudaMemcpy(saved[k], e->field, e->elem * e->Np, cudaMemcpyDeviceToDevice);
+        cudaError_t ce = cudaMalloc(&saved[k], e->elem * e->Np);
+        if (ce == cudaSuccess)
+            ce = cudaMemcpyAsync(saved[k], e->field, e->elem * e->Np, cudaMemcpyDeviceToDevice, e->stream);
+        if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->stream);
         if (ce != cudaSuccess) st = cuda_fail(ce, "bfb_batch_autotune: field copy");
     }
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -903,7 +904,8 @@ BFB_API int bfb_batch_autotune(bfb_batch b, double dt, int flags, int trials, in
     for (int k = 0; k < b->n; ++k) {
         if (!saved[k]) continue;
         bfb_env_s *e = b->envs[k];
-        const cudaError_t ce = cudaMemcpy(e->field, saved[k], e->elem * e->Np, cudaMemcpyDeviceToDevice);
+        cudaError_t ce = cudaMemcpyAsync(e->field, saved[k], e->elem * e->Np, cudaMemcpyDeviceToDevice, e->stream);
+        if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->stream);
         if (ce != cudaSuccess && !st) st = cuda_fail(ce, "bfb_batch_autotune: field restore");
         cudaFree(saved[k]);
     }

@@ -70,13 +70,17 @@ static void axis_factors(int n, int S, double dt, double dx, const double *D, co
     }
 }
 
+// Uploads go through the env's stream and their callers wait for it: a copy
+// from pageable memory on the legacy stream may return before its last bytes
+// are on the device, and kernels on the env's non-blocking stream do not wait
+// for that stream.
 static int upload_table(bfb_env_s *env, void *dst, const std::vector<double> &v) {
     if (env->precision == BFB_FP64) {
-        BFB_CUDA(cudaMemcpy(dst, v.data(), v.size() * sizeof(double), cudaMemcpyHostToDevice));
+        BFB_CUDA(cudaMemcpyAsync(dst, v.data(), v.size() * sizeof(double), cudaMemcpyHostToDevice, env->stream));
     } else {
         std::vector<float> f(v.size());
         for (size_t q = 0; q < v.size(); ++q) f[q] = (float)v[q];
-        BFB_CUDA(cudaMemcpy(dst, f.data(), f.size() * sizeof(float), cudaMemcpyHostToDevice));
+        BFB_CUDA(cudaMemcpyAsync(dst, f.data(), f.size() * sizeof(float), cudaMemcpyHostToDevice, env->stream));
     }
     return BFB_OK;
 }
@@ -93,7 +97,8 @@ static int upload_pitched_table(bfb_env_s *env, void *dst, const std::vector<dou
         for (size_t q = 0; q < v.size(); ++q) f[q] = (float)v[q];
         src = f.data();
     }
-    BFB_CUDA(cudaMemcpy2D(dst, (size_t)env->Lp * eb, src, L * eb, L * eb, rows, cudaMemcpyHostToDevice));
+    BFB_CUDA(cudaMemcpy2DAsync(dst, (size_t)env->Lp * eb, src, L * eb, L * eb, rows, cudaMemcpyHostToDevice,
+                               env->stream));
     return BFB_OK;
 }
 
@@ -204,6 +209,7 @@ static int ensure_factors(bfb_env_s *env, double dt) {
         g[env->S + d] = (double)(float)(gv - g[d]);
     }
     if ((st = upload_table(env, env->g, g))) return st;
+    BFB_CUDA(cudaStreamSynchronize(env->stream));
     env->factors_valid = true;
     env->factor_dt = dt;
     env->epoch++;
@@ -392,16 +398,18 @@ static int bulk_tabulate(bfb_env_s *env, const double *Sr, const double *T, cons
     // (row padding zero, so a whole-array pass leaves padded field entries finite)
     if (!env->bulkA) {
         BFB_CUDA(cudaMalloc(&env->bulkA, env->elem * env->Np));
-        BFB_CUDA(cudaMemset(env->bulkA, 0, env->elem * env->Np));
+        BFB_CUDA(cudaMemsetAsync(env->bulkA, 0, env->elem * env->Np, env->stream));
     }
     if (!env->bulkB) {
         BFB_CUDA(cudaMalloc(&env->bulkB, env->elem * env->Np));
-        BFB_CUDA(cudaMemset(env->bulkB, 0, env->elem * env->Np));
+        BFB_CUDA(cudaMemsetAsync(env->bulkB, 0, env->elem * env->Np, env->stream));
     }
     BFB_CUDA(cudaStreamSynchronize(env->stream));
     int st = upload_pitched_table(env, env->bulkA, A);
+    if (!st) st = upload_pitched_table(env, env->bulkB, B);
     if (st) return st;
-    return upload_pitched_table(env, env->bulkB, B);
+    BFB_CUDA(cudaStreamSynchronize(env->stream));
+    return BFB_OK;
 }
 
 }  // namespace bfb
@@ -485,10 +493,6 @@ BFB_API int bfb_create(bfb_env *out, int nx, int ny, int nz, int n_substrates, d
     alloc(&env->g, env->elem * 2 * n_substrates);
     alloc((void **)&env->d_mask, n_substrates);
     alloc((void **)&env->d_err, sizeof(int));
-    if (!st) {
-        cudaError_t e = cudaMemset(env->d_err, 0, sizeof(int));
-        if (e != cudaSuccess) st = cuda_fail(e, "cudaMemset");
-    }
     if (!st) encode_field_maps(env);
     if (!st) {
         cudaError_t e = cudaStreamCreateWithFlags(&env->own_stream, cudaStreamNonBlocking);
@@ -496,8 +500,10 @@ BFB_API int bfb_create(bfb_env *out, int nx, int ny, int nz, int n_substrates, d
         env->stream = env->own_stream;
     }
     if (!st) {
-        cudaError_t e = cudaMemset(env->field, 0, env->elem * env->Np);
-        if (e == cudaSuccess) e = cudaMemset(env->d_mask, 0, n_substrates);
+        cudaError_t e = cudaMemsetAsync(env->field, 0, env->elem * env->Np, env->stream);
+        if (e == cudaSuccess) e = cudaMemsetAsync(env->d_mask, 0, n_substrates, env->stream);
+        if (e == cudaSuccess) e = cudaMemsetAsync(env->d_err, 0, sizeof(int), env->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(env->stream);
         if (e != cudaSuccess) st = cuda_fail(e, "cudaMemset");
     }
     if (st) {
@@ -781,7 +787,7 @@ static int dirichlet_install(bfb_env_s *env, const std::vector<double> *faces_ho
     for (int f = 0; f < 6; ++f)
         if (!env->faces[f]) {
             BFB_CUDA(cudaMalloc(&env->faces[f], env->elem * fsz[f] * S));
-            BFB_CUDA(cudaMemset(env->faces[f], 0, env->elem * fsz[f] * S));
+            BFB_CUDA(cudaMemsetAsync(env->faces[f], 0, env->elem * fsz[f] * S, env->stream));
         }
     BFB_CUDA(cudaStreamSynchronize(env->stream));
     if (faces_host)
@@ -789,7 +795,8 @@ static int dirichlet_install(bfb_env_s *env, const std::vector<double> *faces_ho
             int st = upload_table(env, env->faces[f], faces_host[f]);
             if (st) return st;
         }
-    BFB_CUDA(cudaMemcpy(env->d_mask, bits.data(), S, cudaMemcpyHostToDevice));
+    BFB_CUDA(cudaMemcpyAsync(env->d_mask, bits.data(), S, cudaMemcpyHostToDevice, env->stream));
+    BFB_CUDA(cudaStreamSynchronize(env->stream));
     env->dir_any = any != 0;
     env->epoch++;
     return BFB_OK;
