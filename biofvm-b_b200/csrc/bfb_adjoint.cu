@@ -832,6 +832,26 @@ __global__ void cells_adjoint_kernel(T *__restrict__ lam, T *__restrict__ w, con
     w[fe] = v;
 }
 
+// Chain rule of one agent's constants to its rates, sorted order to list order:
+// temp1 = c S rho*, temp2 = 1 + c S + c U, c = dt*volume/dV
+// (set_internal_uptake_constants). Inactive agents keep the zeros set before.
+__global__ void agent_rates_adjoint_kernel(int n_active, int S, const int *__restrict__ order,
+                                           const double *__restrict__ gt1, const double *__restrict__ gt2,
+                                           const double *__restrict__ vol, const double *__restrict__ sec,
+                                           const double *__restrict__ sat, double dt, double dV,
+                                           double *__restrict__ gsec, double *__restrict__ gupt,
+                                           double *__restrict__ gsat) {
+    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= (long long)n_active * S) return;
+    const int r = (int)(e / S), d = (int)(e - (long long)r * S);
+    const int a = order[r];
+    const size_t la = (size_t)a * S + d;
+    const double cc = __ddiv_rn(__dmul_rn(dt, vol[a]), dV);
+    gsec[la] = __dadd_rn(__dmul_rn(__dmul_rn(gt1[e], cc), sat[la]), __dmul_rn(gt2[e], cc));
+    gupt[la] = __dmul_rn(gt2[e], cc);
+    gsat[la] = __dmul_rn(__dmul_rn(gt1[e], cc), sec[la]);
+}
+
 }  // namespace bfb
 
 // ---------------------------------------------------------------------------
@@ -1066,7 +1086,9 @@ int adjoint_run(bfb_env_s *env, double dt, int n_steps, int flags, int K, const 
     const bool padded = env->Lp != env->nz * S;
     T *head = nullptr;
     T *vkeep = nullptr;
-    double *part = nullptr, *gacc = nullptr, *gt1 = nullptr, *gt2 = nullptr, *coef = nullptr;
+    double *part = nullptr, *gacc = nullptr, *gt1 = nullptr, *gt2 = nullptr, *coef = nullptr, *grates = nullptr;
+    const bool want_rates = (gsec || gupt || gsat) && cells;
+    const size_t nlist = (size_t)env->n_agents * S;
     auto carve = [&](Carve &c) {
         for (auto &p : ckpt) c.take(&p, fb);
         for (auto *v : {&S1, &S2, &W})
@@ -1087,6 +1109,7 @@ int adjoint_run(bfb_env_s *env, double dt, int n_steps, int flags, int K, const 
         c.take(&vkeep, sizeof(T) * occ * K);
         c.take(&gt1, sizeof(double) * nact);
         c.take(&gt2, sizeof(double) * nact);
+        c.take(&grates, want_rates ? sizeof(double) * 3 * nlist : 0);
     };
     Carve sizing;
     carve(sizing);
@@ -1221,13 +1244,12 @@ int adjoint_run(bfb_env_s *env, double dt, int n_steps, int flags, int K, const 
     // ---- gradients to the caller
     std::vector<double> acc(2 * S);
     BFB_CUDA(cudaMemcpyAsync(acc.data(), gacc, sizeof(double) * 2 * S, cudaMemcpyDeviceToHost, st));
-    std::vector<double> h1(nact), h2(nact);
-    std::vector<int> order(env->n_active);
-    if (nact) {
-        BFB_CUDA(cudaMemcpyAsync(h1.data(), gt1, sizeof(double) * nact, cudaMemcpyDeviceToHost, st));
-        BFB_CUDA(cudaMemcpyAsync(h2.data(), gt2, sizeof(double) * nact, cudaMemcpyDeviceToHost, st));
-        BFB_CUDA(cudaMemcpyAsync(order.data(), env->ag_order, sizeof(int) * env->n_active, cudaMemcpyDeviceToHost,
-                                 st));
+    if (want_rates && env->rates_known) {
+        BFB_CUDA(cudaMemsetAsync(grates, 0, sizeof(double) * 3 * nlist, st));
+        agent_rates_adjoint_kernel<<<(unsigned)((nact + 255) / 256), 256, 0, st>>>(
+            env->n_active, S, env->ag_order, gt1, gt2, env->ag_vol, env->ag_sec, env->ag_sat, env->agent_dt,
+            (env->dx * env->dx) * env->dx, grates, grates + nlist, grates + 2 * nlist);
+        BFB_CUDA(cudaGetLastError());
     }
     BFB_CUDA(cudaStreamSynchronize(st));
     int herr = 0;
@@ -1238,26 +1260,17 @@ int adjoint_run(bfb_env_s *env, double dt, int n_steps, int flags, int K, const 
         if (gD) gD[d] = kD * acc[d];
         if (gL) gL[d] = kL * acc[S + d];
     }
-    // temp1 = c S rho*, temp2 = 1 + c S + c U, c = dt*volume/dV (set_internal_uptake_constants)
-    const size_t nlist = (size_t)env->n_agents * S;
-    if (gsec) std::fill(gsec, gsec + nlist, 0.0);
-    if (gupt) std::fill(gupt, gupt + nlist, 0.0);
-    if (gsat) std::fill(gsat, gsat + nlist, 0.0);
-    if ((gsec || gupt || gsat) && cells) {
-        if (env->h_sec.empty())
-            return fail(BFB_ERR_STATE, "adjoint: agents were set from cached constants; rates are unknown");
-        const double dV = (env->dx * env->dx) * env->dx;
-        for (int q = 0; q < env->n_active; ++q) {
-            const int a = order[q];
-            const double cc = env->agent_dt * env->h_vol[a] / dV;
-            for (int d = 0; d < S; ++d) {
-                const size_t qa = (size_t)q * S + d, la = (size_t)a * S + d;
-                if (gsec) gsec[la] = h1[qa] * cc * env->h_sat[la] + h2[qa] * cc;
-                if (gupt) gupt[la] = h2[qa] * cc;
-                if (gsat) gsat[la] = h1[qa] * cc * env->h_sec[la];
-            }
-        }
+    double *const rates_out[3] = {gsec, gupt, gsat};
+    for (int q = 0; q < 3; ++q) {
+        if (!rates_out[q]) continue;
+        if (want_rates && env->rates_known)
+            BFB_CUDA(cudaMemcpyAsync(rates_out[q], grates + q * nlist, sizeof(double) * nlist, cudaMemcpyDeviceToHost, st));
+        else
+            std::fill(rates_out[q], rates_out[q] + nlist, 0.0);
     }
+    BFB_CUDA(cudaStreamSynchronize(st));
+    if (want_rates && !env->rates_known)
+        return fail(BFB_ERR_STATE, "adjoint: agents were set from cached constants; rates are unknown");
     return BFB_OK;
 }
 

@@ -2,8 +2,10 @@
 #include "bfb_aux.cuh"
 
 #include <cub/cub.cuh>
+#include <thrust/iterator/counting_iterator.h>
 
 #include <algorithm>
+#include <type_traits>
 
 namespace bfb {
 
@@ -91,14 +93,14 @@ __device__ __forceinline__ int bin_axis(double p, double lo, double hi, double h
     return v;
 }
 
-__global__ void bin_agents_kernel(int n, int S, const double *__restrict__ pos, const double *__restrict__ vol,
-                                  const double *__restrict__ sec, const double *__restrict__ upt,
-                                  const double *__restrict__ sat, double dt, BinGeom g, int *__restrict__ voxel,
-                                  double *__restrict__ t1, double *__restrict__ t2) {
+// The voxel of each agent, and the (key, list index) pairs to sort: the voxel,
+// or V for an inactive agent, so that those sort past every segment.
+__global__ void bin_agents_kernel(int n, const double *__restrict__ pos, const uint8_t *__restrict__ active, BinGeom g,
+                                  int *__restrict__ voxel, int *__restrict__ key, int *__restrict__ idx) {
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= n) return;
-    const double x = pos[3 * a], y = pos[3 * a + 1], z = pos[3 * a + 2];
-    int idx = 0;  // a freshly created agent's current_voxel_index
+    const double x = pos[3 * (size_t)a], y = pos[3 * (size_t)a + 1], z = pos[3 * (size_t)a + 2];
+    int v = 0;  // a freshly created agent's current_voxel_index
     const bool valid = !(x < g.lo[0] || x > g.hi[0] || y < g.lo[1] || y > g.hi[1] || z < g.lo[2] || z > g.hi[2]);
     if (valid) {
         const int xi = bin_axis(x, g.lo[0], g.hi[0], g.h[0]);
@@ -106,29 +108,68 @@ __global__ void bin_agents_kernel(int n, int S, const double *__restrict__ pos, 
         const int zi = bin_axis(z, g.lo[2], g.hi[2], g.h[2]);
         const int lny = (int)__ddiv_rn(__dsub_rn(g.hi[1], g.lo[1]), g.h[1]);
         const int lnz = (int)__ddiv_rn(__dsub_rn(g.hi[2], g.lo[2]), g.h[2]);
-        idx = xi * lny * lnz + yi * lnz + zi;
-        if (idx < 0) idx = 0;
-        if (idx >= g.V) idx = g.V - 1;
+        v = xi * lny * lnz + yi * lnz + zi;
+        if (v < 0) v = 0;
+        if (v >= g.V) v = g.V - 1;
     }
-    voxel[a] = idx;
-    const double c = __ddiv_rn(__dmul_rn(dt, vol[a]), g.dV);
-    for (int d = 0; d < S; ++d) {
-        const size_t e = (size_t)a * S + d;
-        t1[e] = __dmul_rn(__dmul_rn(sec[e], sat[e]), c);
-        t2[e] = __fma_rn(c, upt[e], __fma_rn(c, sec[e], 1.0));
-    }
+    voxel[a] = v;
+    key[a] = !active || active[a] ? v : g.V;
+    idx[a] = a;
 }
 
+__global__ void key_agents_kernel(int n, const int *__restrict__ voxel, const uint8_t *__restrict__ active, int V,
+                                  int *__restrict__ key, int *__restrict__ idx) {
+    const int a = blockIdx.x * blockDim.x + threadIdx.x;
+    if (a >= n) return;
+    key[a] = !active || active[a] ? voxel[a] : V;
+    idx[a] = a;
+}
+
+// Of the sorted keys: head[r] = 1 where a voxel's segment starts, and
+// counts[1] = the number of active agents (keys below V; zeroed before).
+__global__ void segment_heads_kernel(int n, const int *__restrict__ key, int V, uint8_t *__restrict__ head,
+                                     int *__restrict__ counts) {
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= n) return;
+    const int k = key[r];
+    head[r] = k < V && (r == 0 || key[r - 1] != k);
+    if (k < V && (r == n - 1 || key[r + 1] >= V)) counts[1] = r + 1;
+}
+
+// seg_voxel of each segment and the end of the last one; counts = {segments, active agents}.
+__global__ void segment_ends_kernel(const int *__restrict__ key, const int *__restrict__ counts,
+                                    int *__restrict__ seg_start, int *__restrict__ seg_voxel) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x, n_occ = counts[0];
+    if (s < n_occ) seg_voxel[s] = key[seg_start[s]];
+    if (s == n_occ) seg_start[s] = counts[1];
+}
+
+// The constants of the sorted agents, from the rates ...
 template <typename T>
-__global__ void gather_constants_kernel(int n_active, int S, const int *__restrict__ order,
+__global__ void agent_constants_kernel(const int *__restrict__ counts, int S, const int *__restrict__ order,
+                                       const double *__restrict__ vol, const double *__restrict__ sec,
+                                       const double *__restrict__ upt, const double *__restrict__ sat, double dt,
+                                       double dV, T *__restrict__ o1, T *__restrict__ o2) {
+    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= (long long)counts[1] * S) return;
+    const int r = (int)(e / S), d = (int)(e - (long long)r * S);
+    const int a = order[r];
+    const size_t q = (size_t)a * S + d;
+    const double c = __ddiv_rn(__dmul_rn(dt, vol[a]), dV);
+    o1[e] = (T)__dmul_rn(__dmul_rn(sec[q], sat[q]), c);
+    o2[e] = (T)__fma_rn(c, upt[q], __fma_rn(c, sec[q], 1.0));
+}
+// ... or as given.
+template <typename T>
+__global__ void gather_constants_kernel(const int *__restrict__ counts, int S, const int *__restrict__ order,
                                         const double *__restrict__ t1, const double *__restrict__ t2,
                                         T *__restrict__ o1, T *__restrict__ o2) {
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (long long)n_active * S) return;
-    const int r = (int)(e / S), d = (int)(e % S);
-    const int a = order[r];
-    o1[e] = (T)t1[(size_t)a * S + d];
-    o2[e] = (T)t2[(size_t)a * S + d];
+    if (e >= (long long)counts[1] * S) return;
+    const int r = (int)(e / S), d = (int)(e - (long long)r * S);
+    const size_t q = (size_t)order[r] * S + d;
+    o1[e] = (T)t1[q];
+    o2[e] = (T)t2[q];
 }
 
 // BioFVM_basic_agent.cpp:291-296 for all agents of one voxel, in list order.
@@ -154,125 +195,132 @@ __global__ void cells_kernel(T *__restrict__ f, int S, int nz, int Lp, int n_occ
 }
 
 void agents_free(bfb_env_s *env) {
-    cudaFree(env->agent_voxel);
-    cudaFree(env->seg_start);
-    cudaFree(env->seg_voxel);
-    cudaFree(env->ag_t1);
-    cudaFree(env->ag_t2);
-    cudaFree(env->ag_order);
-    env->ag_order = nullptr;
-    env->agent_voxel = env->seg_start = env->seg_voxel = nullptr;
-    env->ag_t1 = env->ag_t2 = nullptr;
+    cudaFree(env->ag_ws);
+    env->ag_ws = nullptr;
+    env->ag_ws_bytes = 0;
     env->n_agents = env->n_occ = env->n_active = 0;
+    env->rates_known = false;
 }
 
 namespace {
-struct DevBuf {
-    void *p = nullptr;
-    ~DevBuf() { cudaFree(p); }
-    cudaError_t alloc(size_t bytes) { return cudaMalloc(&p, bytes ? bytes : 1); }
-    template <typename U>
-    U *as() { return static_cast<U *>(p); }
+
+// The scratch of one agents_build call, in the env's agent block.
+struct AgentScratch {
+    double *pos, *t1, *t2;  // positions; constants as given (in the rates' place)
+    uint8_t *active, *head;
+    int *key, *key_sorted, *idx, *counts;
+    void *tmp;
+    size_t sort_bytes, select_bytes;
 };
-}  // namespace
 
-// Sort the active agents by voxel (stable: list order within a voxel) and
-// build the per-voxel segments the cells kernel walks. d_vox/d_t1/d_t2 are
-// device arrays in list order (d_t1/d_t2 FP64, [n][S]); active may be NULL.
-static int index_agents(bfb_env_s *env, int n, const int *d_vox, const double *d_t1, const double *d_t2,
-                        const uint8_t *active) {
-    const int S = env->S;
-    cudaStream_t s = env->stream;
-    std::vector<int> h_vox(n);
-    BFB_CUDA(cudaMemcpyAsync(h_vox.data(), d_vox, sizeof(int) * n, cudaMemcpyDeviceToHost, s));
-    BFB_CUDA(cudaStreamSynchronize(s));
-    std::vector<int> keys, idx;
-    keys.reserve(n);
-    idx.reserve(n);
-    for (int a = 0; a < n; ++a) {
-        if (!active || active[a]) {
-            if (h_vox[a] < 0 || h_vox[a] >= env->V) return fail(BFB_ERR_INVALID_ARG, "agent voxel index out of range");
-            keys.push_back(h_vox[a]);
-            idx.push_back(a);
-        }
-    }
-    const int na = (int)keys.size();
-    env->n_active = na;
-    if (na == 0) return BFB_OK;
-    DevBuf d_keys, d_keys_sorted, d_idx, d_idx_sorted, d_unique, d_counts, d_nruns, d_tmp;
-    BFB_CUDA(d_keys.alloc(sizeof(int) * na));
-    BFB_CUDA(d_keys_sorted.alloc(sizeof(int) * na));
-    BFB_CUDA(d_idx.alloc(sizeof(int) * na));
-    BFB_CUDA(d_idx_sorted.alloc(sizeof(int) * na));
-    BFB_CUDA(d_unique.alloc(sizeof(int) * na));
-    BFB_CUDA(d_counts.alloc(sizeof(int) * na));
-    BFB_CUDA(d_nruns.alloc(sizeof(int)));
-    BFB_CUDA(cudaMemcpyAsync(d_keys.p, keys.data(), sizeof(int) * na, cudaMemcpyHostToDevice, s));
-    BFB_CUDA(cudaMemcpyAsync(d_idx.p, idx.data(), sizeof(int) * na, cudaMemcpyHostToDevice, s));
-
-    // Stable LSD radix sort by voxel: agents of one voxel stay in list order.
+// Lays the env's agent arrays and the scratch for n agents out in its agent
+// block, which is kept between calls and grows when it must. A program sets its
+// agents once per mechanics step; allocating and freeing seventeen arrays on
+// each call (every cudaFree waits for the device) took most of a call's time:
+// 40,000 agents x 4 substrates 4.3 -> 0.41 ms a call, 100,000 x 8 12 -> 1.3,
+// now bound by the rates crossing the host link from pageable memory.
+int agents_layout(bfb_env_s *env, int n, bool rates, AgentScratch *w) {
+    const size_t N = (size_t)n, nS = N * env->S;
     int end_bit = 1;
-    while (end_bit < 31 && (1LL << end_bit) < env->V) ++end_bit;
-    size_t tmp_sort = 0, tmp_rle = 0;
-    BFB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp_sort, d_keys.as<int>(), d_keys_sorted.as<int>(),
-                                             d_idx.as<int>(), d_idx_sorted.as<int>(), na, 0, end_bit, s));
-    BFB_CUDA(cub::DeviceRunLengthEncode::Encode(nullptr, tmp_rle, d_keys_sorted.as<int>(), d_unique.as<int>(),
-                                                d_counts.as<int>(), d_nruns.as<int>(), na, s));
-    BFB_CUDA(d_tmp.alloc(std::max(tmp_sort, tmp_rle)));
-    BFB_CUDA(cub::DeviceRadixSort::SortPairs(d_tmp.p, tmp_sort, d_keys.as<int>(), d_keys_sorted.as<int>(),
-                                             d_idx.as<int>(), d_idx_sorted.as<int>(), na, 0, end_bit, s));
-    BFB_CUDA(cub::DeviceRunLengthEncode::Encode(d_tmp.p, tmp_rle, d_keys_sorted.as<int>(), d_unique.as<int>(),
-                                                d_counts.as<int>(), d_nruns.as<int>(), na, s));
-    int n_occ = 0;
-    BFB_CUDA(cudaMemcpyAsync(&n_occ, d_nruns.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-    BFB_CUDA(cudaStreamSynchronize(s));
-    std::vector<int> counts(n_occ), starts(n_occ + 1, 0);
-    BFB_CUDA(cudaMemcpy(counts.data(), d_counts.p, sizeof(int) * n_occ, cudaMemcpyDeviceToHost));
-    for (int q = 0; q < n_occ; ++q) starts[q + 1] = starts[q] + counts[q];
-    BFB_CUDA(cudaMalloc(&env->seg_start, sizeof(int) * (n_occ + 1)));
-    BFB_CUDA(cudaMalloc(&env->seg_voxel, sizeof(int) * std::max(1, n_occ)));
-    BFB_CUDA(cudaMemcpyAsync(env->seg_start, starts.data(), sizeof(int) * (n_occ + 1), cudaMemcpyHostToDevice, s));
-    BFB_CUDA(cudaMemcpyAsync(env->seg_voxel, d_unique.p, sizeof(int) * n_occ, cudaMemcpyDeviceToDevice, s));
-    env->n_occ = n_occ;
-
-    BFB_CUDA(cudaMalloc(&env->ag_order, sizeof(int) * na));
-    BFB_CUDA(cudaMemcpyAsync(env->ag_order, d_idx_sorted.p, sizeof(int) * na, cudaMemcpyDeviceToDevice, s));
-    BFB_CUDA(cudaMalloc(&env->ag_t1, env->elem * (size_t)na * S));
-    BFB_CUDA(cudaMalloc(&env->ag_t2, env->elem * (size_t)na * S));
-    const long long tot = (long long)na * S;
-    const unsigned gb = (unsigned)((tot + 255) / 256);
-    if (env->precision == BFB_FP64)
-        gather_constants_kernel<double><<<gb, 256, 0, s>>>(na, S, d_idx_sorted.as<int>(), d_t1, d_t2,
-                                                           (double *)env->ag_t1, (double *)env->ag_t2);
-    else
-        gather_constants_kernel<float><<<gb, 256, 0, s>>>(na, S, d_idx_sorted.as<int>(), d_t1, d_t2,
-                                                          (float *)env->ag_t1, (float *)env->ag_t2);
-    BFB_CUDA(cudaGetLastError());
-    BFB_CUDA(cudaStreamSynchronize(s));  // temporaries are freed on return
+    while (end_bit < 31 && (1LL << end_bit) <= env->V) ++end_bit;
+    env->ag_end_bit = end_bit;  // keys 0 .. V
+    w->sort_bytes = w->select_bytes = 0;
+    BFB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, w->sort_bytes, (const int *)nullptr, (int *)nullptr,
+                                             (const int *)nullptr, (int *)nullptr, n, 0, end_bit, env->stream));
+    BFB_CUDA(cub::DeviceSelect::Flagged(nullptr, w->select_bytes, thrust::counting_iterator<int>(0),
+                                        (const uint8_t *)nullptr, (int *)nullptr, (int *)nullptr, n, env->stream));
+    char *base = nullptr;
+    size_t off = 0;
+    auto take = [&](auto **p, size_t bytes) {
+        *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(base ? base + off : nullptr);
+        off += (std::max<size_t>(bytes, 1) + 255) / 256 * 256;
+    };
+    auto lay = [&]() {
+        off = 0;
+        take(&env->agent_voxel, sizeof(int) * N);
+        take(&env->seg_start, sizeof(int) * (N + 1));
+        take(&env->seg_voxel, sizeof(int) * N);
+        take(&env->ag_order, sizeof(int) * N);
+        take((char **)&env->ag_t1, env->elem * nS);
+        take((char **)&env->ag_t2, env->elem * nS);
+        if (rates) {
+            take(&env->ag_vol, sizeof(double) * N);
+            take(&env->ag_sec, sizeof(double) * nS);
+            take(&env->ag_upt, sizeof(double) * nS);
+            take(&env->ag_sat, sizeof(double) * nS);
+            take(&w->pos, sizeof(double) * 3 * N);
+        } else {
+            take(&w->t1, sizeof(double) * nS);
+            take(&w->t2, sizeof(double) * nS);
+        }
+        take(&w->active, N);
+        take(&w->head, N);
+        take(&w->key, sizeof(int) * N);
+        take(&w->key_sorted, sizeof(int) * N);
+        take(&w->idx, sizeof(int) * N);
+        take(&w->counts, sizeof(int) * 2);
+        take((char **)&w->tmp, std::max(w->sort_bytes, w->select_bytes));
+    };
+    lay();
+    if (off > env->ag_ws_bytes) {
+        const size_t want = off + off / 4;  // agents divide
+        agents_free(env);
+        BFB_CUDA(cudaMalloc(&env->ag_ws, want));
+        env->ag_ws_bytes = want;
+    }
+    base = static_cast<char *>(env->ag_ws);
+    lay();
     return BFB_OK;
 }
 
+// Sorts the active agents by voxel (stable: list order within a voxel) and
+// builds the per-voxel segments the cells kernel walks, from w.key / w.idx.
+int agents_sort(bfb_env_s *env, int n, AgentScratch &w) {
+    cudaStream_t s = env->stream;
+    BFB_CUDA(cudaMemsetAsync(w.counts, 0, 2 * sizeof(int), s));
+    BFB_CUDA(cub::DeviceRadixSort::SortPairs(w.tmp, w.sort_bytes, w.key, w.key_sorted, w.idx, env->ag_order, n, 0,
+                                             env->ag_end_bit, s));
+    segment_heads_kernel<<<(n + 255) / 256, 256, 0, s>>>(n, w.key_sorted, (int)env->V, w.head, w.counts);
+    BFB_CUDA(cudaGetLastError());
+    BFB_CUDA(cub::DeviceSelect::Flagged(w.tmp, w.select_bytes, thrust::counting_iterator<int>(0), w.head,
+                                        env->seg_start, w.counts, n, s));
+    segment_ends_kernel<<<(n + 256) / 256, 256, 0, s>>>(w.key_sorted, w.counts, env->seg_start, env->seg_voxel);
+    BFB_CUDA(cudaGetLastError());
+    return BFB_OK;
+}
+
+// Waits for the build and takes the counts the launches are sized by.
+int agents_finish(bfb_env_s *env, const AgentScratch &w) {
+    int counts[2] = {0, 0};
+    BFB_CUDA(cudaMemcpyAsync(counts, w.counts, sizeof(counts), cudaMemcpyDeviceToHost, env->stream));
+    BFB_CUDA(cudaStreamSynchronize(env->stream));
+    env->n_occ = counts[0];
+    env->n_active = counts[1];
+    return BFB_OK;
+}
+
+// No kernel may still read the agent arrays: the env's own stream is idle
+// (bfb_set_agents waits for it), a batch's streams may not be.
+int agents_quiesce(bfb_env_s *env) {
+    if (env->batched) BFB_CUDA(cudaDeviceSynchronize());
+    env->n_agents = env->n_occ = env->n_active = 0;
+    env->rates_known = false;
+    return BFB_OK;
+}
+
+}  // namespace
+
 int agents_build(bfb_env_s *env, int n, const double *pos, const double *volume, const double *sec,
                  const double *upt, const double *sat, const uint8_t *active, double dt) {
-    agents_free(env);
-    if (n == 0) return BFB_OK;
+    int st = agents_quiesce(env);
+    if (st || n == 0) return st;
     const int S = env->S;
+    const size_t nS = (size_t)n * S;
     cudaStream_t s = env->stream;
-    DevBuf d_pos, d_vol, d_sec, d_upt, d_sat, d_t1, d_t2;
-    BFB_CUDA(d_pos.alloc(sizeof(double) * 3 * n));
-    BFB_CUDA(d_vol.alloc(sizeof(double) * n));
-    BFB_CUDA(d_sec.alloc(sizeof(double) * n * S));
-    BFB_CUDA(d_upt.alloc(sizeof(double) * n * S));
-    BFB_CUDA(d_sat.alloc(sizeof(double) * n * S));
-    BFB_CUDA(d_t1.alloc(sizeof(double) * n * S));
-    BFB_CUDA(d_t2.alloc(sizeof(double) * n * S));
-    BFB_CUDA(cudaMalloc(&env->agent_voxel, sizeof(int) * n));
-    BFB_CUDA(cudaMemcpyAsync(d_pos.p, pos, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, s));
-    BFB_CUDA(cudaMemcpyAsync(d_vol.p, volume, sizeof(double) * n, cudaMemcpyHostToDevice, s));
-    BFB_CUDA(cudaMemcpyAsync(d_sec.p, sec, sizeof(double) * n * S, cudaMemcpyHostToDevice, s));
-    BFB_CUDA(cudaMemcpyAsync(d_upt.p, upt, sizeof(double) * n * S, cudaMemcpyHostToDevice, s));
-    BFB_CUDA(cudaMemcpyAsync(d_sat.p, sat, sizeof(double) * n * S, cudaMemcpyHostToDevice, s));
-
+    AgentScratch w;
+    if ((st = agents_layout(env, n, true, &w))) return st;
+    BFB_CUDA(cudaMemcpyAsync(w.pos, pos, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, s));
+    if (active) BFB_CUDA(cudaMemcpyAsync(w.active, active, n, cudaMemcpyHostToDevice, s));
     BinGeom g;
     for (int a = 0; a < 3; ++a) {
         g.lo[a] = env->bbox[a];
@@ -281,29 +329,63 @@ int agents_build(bfb_env_s *env, int n, const double *pos, const double *volume,
     }
     g.V = (int)env->V;
     g.dV = (env->dx * env->dx) * env->dx;
-    bin_agents_kernel<<<(n + 127) / 128, 128, 0, s>>>(n, S, d_pos.as<double>(), d_vol.as<double>(),
-                                                      d_sec.as<double>(), d_upt.as<double>(), d_sat.as<double>(), dt,
-                                                      g, env->agent_voxel, d_t1.as<double>(), d_t2.as<double>());
+    bin_agents_kernel<<<(n + 127) / 128, 128, 0, s>>>(n, w.pos, active ? w.active : nullptr, g, env->agent_voxel, w.key,
+                                                      w.idx);
     BFB_CUDA(cudaGetLastError());
     env->n_agents = n;
-    return index_agents(env, n, env->agent_voxel, d_t1.as<double>(), d_t2.as<double>(), active);
+    if ((st = agents_sort(env, n, w))) return st;
+    // the rates cross the host link while the sort runs
+    BFB_CUDA(cudaMemcpyAsync(env->ag_vol, volume, sizeof(double) * n, cudaMemcpyHostToDevice, s));
+    BFB_CUDA(cudaMemcpyAsync(env->ag_sec, sec, sizeof(double) * nS, cudaMemcpyHostToDevice, s));
+    BFB_CUDA(cudaMemcpyAsync(env->ag_upt, upt, sizeof(double) * nS, cudaMemcpyHostToDevice, s));
+    BFB_CUDA(cudaMemcpyAsync(env->ag_sat, sat, sizeof(double) * nS, cudaMemcpyHostToDevice, s));
+    const unsigned gb = (unsigned)((nS + 255) / 256);
+    if (env->precision == BFB_FP64)
+        agent_constants_kernel<double><<<gb, 256, 0, s>>>(w.counts, S, env->ag_order, env->ag_vol, env->ag_sec,
+                                                          env->ag_upt, env->ag_sat, dt, g.dV, (double *)env->ag_t1,
+                                                          (double *)env->ag_t2);
+    else
+        agent_constants_kernel<float><<<gb, 256, 0, s>>>(w.counts, S, env->ag_order, env->ag_vol, env->ag_sec,
+                                                         env->ag_upt, env->ag_sat, dt, g.dV, (float *)env->ag_t1,
+                                                         (float *)env->ag_t2);
+    BFB_CUDA(cudaGetLastError());
+    if ((st = agents_finish(env, w))) return st;
+    env->rates_known = true;
+    return BFB_OK;
 }
 
 int agents_build_constants(bfb_env_s *env, int n, const int *voxel, const double *t1, const double *t2,
                            const uint8_t *active) {
-    agents_free(env);
-    if (n == 0) return BFB_OK;
+    int st = agents_quiesce(env);
+    if (st || n == 0) return st;
     const int S = env->S;
+    const size_t nS = (size_t)n * S;
     cudaStream_t s = env->stream;
-    DevBuf d_t1, d_t2;
-    BFB_CUDA(d_t1.alloc(sizeof(double) * n * S));
-    BFB_CUDA(d_t2.alloc(sizeof(double) * n * S));
-    BFB_CUDA(cudaMalloc(&env->agent_voxel, sizeof(int) * n));
+    AgentScratch w;
+    if ((st = agents_layout(env, n, false, &w))) return st;
     BFB_CUDA(cudaMemcpyAsync(env->agent_voxel, voxel, sizeof(int) * n, cudaMemcpyHostToDevice, s));
-    BFB_CUDA(cudaMemcpyAsync(d_t1.p, t1, sizeof(double) * n * S, cudaMemcpyHostToDevice, s));
-    BFB_CUDA(cudaMemcpyAsync(d_t2.p, t2, sizeof(double) * n * S, cudaMemcpyHostToDevice, s));
     env->n_agents = n;
-    return index_agents(env, n, env->agent_voxel, d_t1.as<double>(), d_t2.as<double>(), active);
+    for (int a = 0; a < n; ++a)
+        if ((!active || active[a]) && (voxel[a] < 0 || voxel[a] >= env->V)) {
+            BFB_CUDA(cudaStreamSynchronize(s));
+            return fail(BFB_ERR_INVALID_ARG, "agent voxel index out of range");
+        }
+    if (active) BFB_CUDA(cudaMemcpyAsync(w.active, active, n, cudaMemcpyHostToDevice, s));
+    key_agents_kernel<<<(n + 127) / 128, 128, 0, s>>>(n, env->agent_voxel, active ? w.active : nullptr, (int)env->V,
+                                                      w.key, w.idx);
+    BFB_CUDA(cudaGetLastError());
+    if ((st = agents_sort(env, n, w))) return st;
+    BFB_CUDA(cudaMemcpyAsync(w.t1, t1, sizeof(double) * nS, cudaMemcpyHostToDevice, s));
+    BFB_CUDA(cudaMemcpyAsync(w.t2, t2, sizeof(double) * nS, cudaMemcpyHostToDevice, s));
+    const unsigned gb = (unsigned)((nS + 255) / 256);
+    if (env->precision == BFB_FP64)
+        gather_constants_kernel<double><<<gb, 256, 0, s>>>(w.counts, S, env->ag_order, w.t1, w.t2,
+                                                           (double *)env->ag_t1, (double *)env->ag_t2);
+    else
+        gather_constants_kernel<float><<<gb, 256, 0, s>>>(w.counts, S, env->ag_order, w.t1, w.t2, (float *)env->ag_t1,
+                                                          (float *)env->ag_t2);
+    BFB_CUDA(cudaGetLastError());
+    return agents_finish(env, w);
 }
 
 int launch_cells(bfb_env_s *env, cudaStream_t s) {

@@ -13,8 +13,8 @@ int launch_convert_d2f_rows(const double *src, float *dst, long long rows, int L
 int launch_convert_f2d_rows(const float *src, double *dst, long long rows, int L, int sp, int dp, cudaStream_t s);
 
 // Agents: binning + cached constants (FP64, bit-exact with the reference),
-// then a stable voxel sort and per-voxel segments. All device memory of the
-// previous agent set is released first.
+// then a stable voxel sort and per-voxel segments. The previous agent set is
+// dropped first; its device block is kept for the next.
 int agents_build(bfb_env_s *env, int n, const double *pos, const double *volume, const double *sec,
                  const double *upt, const double *sat, const uint8_t *active, double dt);
 // Same, from the constants an agent already caches (current_voxel_index,

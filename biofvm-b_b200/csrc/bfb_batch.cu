@@ -701,6 +701,7 @@ BFB_API int bfb_batch_create(bfb_batch *out, int n_envs, const bfb_env *envs) {
         bfb_batch_destroy(b);
         return st;
     }
+    for (bfb_env_s *env : b->envs) env->batched = true;
     b->stream = b->own_stream;
     *out = b;
     return BFB_OK;

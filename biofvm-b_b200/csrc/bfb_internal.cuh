@@ -177,9 +177,15 @@ struct bfb_env_s {
     void *ag_t1 = nullptr, *ag_t2 = nullptr;  // [n_active][S] in voxel-sorted, list-stable order
     int n_active = 0;
     int *ag_order = nullptr;             // [n_active]: list index of each sorted agent
-    // rates as given to bfb_set_agents (list order), for the adjoint's chain rule
-    std::vector<double> h_vol, h_sec, h_upt, h_sat;
+    // volumes and rates as given to bfb_set_agents (device, list order; valid
+    // when rates_known), also for the adjoint's chain rule
+    double *ag_vol = nullptr, *ag_sec = nullptr, *ag_upt = nullptr, *ag_sat = nullptr;
+    bool rates_known = false;
     double agent_dt = 0;
+    void *ag_ws = nullptr;               // the block holding all of the above (agents_layout)
+    size_t ag_ws_bytes = 0;
+    int ag_end_bit = 1;                  // key bits of the voxel sort
+    bool batched = false;                // a batch was made over this env: its streams may read the agents
 
     // scratch for reductions
     double *partials = nullptr;

@@ -259,6 +259,35 @@ def test_simulate_launches_and_graph_agree(bfb, oracle, rng, calls):
         assert np.array_equal(env.get_field(), want)
 
 
+@pytest.mark.parametrize("sizes", [(1, 300, 0, 40), (257, 256, 255, 1200, 7)])
+def test_agents_set_again_and_again(bfb, oracle, rng, sizes):
+    """Agent sets of growing and shrinking size on one env (the kept block), with inactive agents
+    and crowded voxels, by rates and by cached constants in turn; FP64 bit for bit."""
+    shape, S = (6, 5, 7), 3
+    want = rng.random((*shape, S))
+    D, lam = log_uniform(rng, 1e2, 1e5, S), log_uniform(rng, 1e-3, 1.0, S)
+    env = make_env(bfb, want, D, lam, bfb.FP64)
+    for q, n in enumerate(sizes):
+        pos = rng.random((n, 3)) * np.array(shape) * 20.0
+        vol = rng.random(n) * 500.0
+        sec, upt, sat = log_uniform(rng, 1e-2, 10.0, (3, n, S))
+        active = (rng.random(n) < (0.0 if q == 3 else 0.8)).astype(np.uint8)
+        vox = oracle.bin_agents(pos, (0.0, 0.0, 0.0, *(20.0 * v for v in shape)), 20.0, shape)
+        t1, t2 = oracle.agent_constants(0.01, 20.0, vol, sec, upt, sat)
+        if q % 2 == 0:
+            env.set_agents(pos, vol, sec, upt, sat, 0.01, active=active)
+        else:
+            env.set_agent_constants(vox, t1, t2, active=active)
+        assert np.array_equal(env.agent_voxels(), vox)
+        env.cells_step(0.01)
+        on = active.astype(bool)
+        if on.any():
+            want = oracle.cells_step(want, vox[on], t1[on], t2[on])
+        assert np.array_equal(env.get_field(), want)
+    with pytest.raises(bfb.BFBError):
+        env.set_agent_constants(np.array([0, 6 * 5 * 7]), np.zeros((2, S)), np.ones((2, S)))
+
+
 def test_agents_random_fp64_and_fp32(bfb, oracle, rng):
     shape, S = (20, 18, 16), 3
     dx, dt = 20.0, 0.01
