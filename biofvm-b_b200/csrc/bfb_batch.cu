@@ -369,6 +369,11 @@ struct bfb_batch_s {
     int n_groups = 1;
     cudaStream_t side[kSide] = {};
     cudaEvent_t fork_ev = nullptr, join_ev[kSide] = {};
+    // staged mode: the envs stepped by their own kernels (chains[c], one after
+    // the other on chain_streams[c]; made when first needed)
+    static constexpr int kMaxChains = 32;
+    std::vector<std::vector<bfb_env>> chains;
+    std::vector<cudaStream_t> chain_streams;
     cudaGraphExec_t graph = nullptr;        // one step
     cudaGraphExec_t graph_multi = nullptr;  // kMultiSteps steps (both built together)
     static constexpr int kMultiSteps = 8;
@@ -387,6 +392,19 @@ int env_run_steps(bfb_env_s *env, double dt, int n, int flags, cudaStream_t s);
 }  // namespace bfb
 
 using namespace bfb;
+
+// Staged mode: envs whose field has at least this many bytes, and all envs of
+// a batch of at most kMaxChains, are stepped by their own kernels, all steps of
+// a graph back to back, instead of sharing stage launches. Those kernels read
+// their arguments from the launch rather than through dependent table reads
+// per tile, need fewer registers and follow one another without a step-wide
+// join; what they cost is a launch per env and stage (about 0.8 us of the GPU's
+// front end), which many small envs do not earn. FP32 with agents, us a step,
+// all shared -> this rule (256 KB, 512 KB, 2 MB and 4 MB measured no better):
+//     8 envs of edges 16-32     114 -> 32      8 of 32-160     163 -> 98
+//    48 of 24-80                334 -> 297    48 of 32-160   1146 -> 982
+//   256 of 16-48                642 -> 614   256 of 32-160   5745 -> 5530
+constexpr long long kOwnChainBytes = 1 << 20;
 
 template <typename T>
 static int batch_upload(bfb_batch_s *b, double dt) {
@@ -465,14 +483,32 @@ static int batch_upload(bfb_batch_s *b, double dt) {
     // whose smallest tile needs more than half the class's largest (at most 4
     // classes per group and path)
     auto warp_of = [](size_t bytes) { return (int)((128 + bytes + 127) / 128 * 128); };
+    // Envs of kOwnChainBytes or more are left out of the shared launches
+    // (group -1) and spread over chains of their own kernels in the same way.
     std::vector<int> group(b->n, 0);
     {
-        b->n_groups = std::min(b->n, (int)bfb_batch_s::kSide);
-        std::vector<int> order(b->n);
-        for (int k = 0; k < b->n; ++k) order[k] = k;
         auto work = [&](int k) { return (double)b->envs[k]->N; };
-        std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return work(x) > work(y); });
-        std::vector<double> load(b->n_groups, 0.0);
+        std::vector<int> order, own;
+        for (int k = 0; k < b->n; ++k)
+            (b->n <= bfb_batch_s::kMaxChains || b->envs[k]->Np * (long long)eb >= kOwnChainBytes ? own : order).push_back(k);
+        auto larger = [&](int x, int y) { return work(x) > work(y); };
+        std::stable_sort(order.begin(), order.end(), larger);
+        std::stable_sort(own.begin(), own.end(), larger);
+        b->n_groups = std::min((int)order.size(), (int)bfb_batch_s::kSide);
+        std::vector<double> load(std::min((int)own.size(), (int)bfb_batch_s::kMaxChains), 0.0);
+        b->chains.assign(load.size(), {});
+        for (int k : own) {
+            const int csel = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+            group[k] = -1;
+            b->chains[csel].push_back(b->envs[k]);
+            load[csel] += work(k);
+        }
+        while (b->chain_streams.size() < b->chains.size()) {
+            cudaStream_t cs = nullptr;
+            BFB_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
+            b->chain_streams.push_back(cs);
+        }
+        load.assign(std::max(1, b->n_groups), 0.0);
         for (int k : order) {
             const int gsel = (int)(std::min_element(load.begin(), load.end()) - load.begin());
             group[k] = gsel;
@@ -513,7 +549,7 @@ static int batch_upload(bfb_batch_s *b, double dt) {
                     hi = end;
                 }
                 const int total = ts[hi] - ts[j];
-                if (total > 0) b->classes[s].push_back({j, hi, bs ? warp_of(bs[ps[j]]) : 0, total, path, grp});
+                if (total > 0 && grp >= 0) b->classes[s].push_back({j, hi, bs ? warp_of(bs[ps[j]]) : 0, total, path, grp});
                 j = hi;
             }
         }
@@ -606,6 +642,26 @@ static int batch_launch_staged(bfb_batch_s *b, int flags, cudaStream_t s) {
     for (int i = 0; i < nside; ++i) {
         BFB_CUDA(cudaEventRecord(b->join_ev[i], b->side[i]));
         BFB_CUDA(cudaStreamWaitEvent(main, b->join_ev[i], 0));
+    }
+    return BFB_OK;
+}
+
+// `steps` steps of the staged mode's chains, forked from and joined to `s`.
+static int batch_launch_chains(bfb_batch_s *b, double dt, int flags, int steps, cudaStream_t s) {
+    if (b->chains.empty()) return BFB_OK;
+    BFB_CUDA(cudaEventRecord(b->fork_ev, s));
+    for (size_t c = 0; c < b->chains.size(); ++c) BFB_CUDA(cudaStreamWaitEvent(b->chain_streams[c], b->fork_ev, 0));
+    for (size_t c = 0; c < b->chains.size(); ++c)
+        for (bfb_env e : b->chains[c]) {
+            const int st = env_run_steps(e, dt, steps, flags, b->chain_streams[c]);
+            if (st) return st;
+        }
+    return BFB_OK;
+}
+static int batch_join_chains(bfb_batch_s *b, cudaStream_t s) {
+    for (size_t c = 0; c < b->chains.size(); ++c) {
+        BFB_CUDA(cudaEventRecord(b->join_ev[0], b->chain_streams[c]));
+        BFB_CUDA(cudaStreamWaitEvent(s, b->join_ev[0], 0));
     }
     return BFB_OK;
 }
@@ -725,6 +781,7 @@ BFB_API int bfb_batch_destroy(bfb_batch b) {
         if (b->side[i]) cudaStreamDestroy(b->side[i]);
         if (b->join_ev[i]) cudaEventDestroy(b->join_ev[i]);
     }
+    for (cudaStream_t cs : b->chain_streams) cudaStreamDestroy(cs);
     if (b->fork_ev) cudaEventDestroy(b->fork_ev);
     delete b;
     return BFB_OK;
@@ -781,10 +838,14 @@ static int batch_capture(bfb_batch_s *b, double dt, int flags, int steps, cudaGr
     int st = BFB_OK;
     if (b->mode == BFB_BATCH_MODE_GRAPH)
         st = batch_launch_graph(b, dt, flags, steps, b->stream);
-    else
+    else {
+        const bool staged = b->mode == BFB_BATCH_MODE_STAGED;
+        if (staged) st = batch_launch_chains(b, dt, flags, steps, b->stream);
         for (int q = 0; q < steps && !st; ++q)
             st = b->precision == BFB_FP64 ? batch_launch<double>(b, flags, b->stream)
                                           : batch_launch<float>(b, flags, b->stream);
+        if (staged && !st) st = batch_join_chains(b, b->stream);
+    }
     cudaError_t e = cudaStreamEndCapture(b->stream, &g);
     if (st) {
         if (g) cudaGraphDestroy(g);
@@ -814,15 +875,13 @@ BFB_API int bfb_batch_simulate(bfb_batch b, double dt, int n_steps, int flags) {
         if (st) return st;
         if (!changed && b->graph_epochs[k] != b->envs[k]->epoch) changed = true;
     }
-    if (changed || !b->graph) {
+    if (changed || (!b->graph && !b->graph_multi)) {
         batch_drop_graph(b);
         int st = b->mode == BFB_BATCH_MODE_GRAPH ? BFB_OK  // the envs' own launches need no tables
                  : b->precision == BFB_FP64     ? batch_upload<double>(b, dt)
                                                 : batch_upload<float>(b, dt);
         if (st) return st;
         for (bfb_env e : b->envs) BFB_CUDA(cudaStreamSynchronize(e->stream));
-        if ((st = batch_capture(b, dt, flags, 1, &b->graph))) return st;
-        if ((st = batch_capture(b, dt, flags, bfb_batch_s::kMultiSteps, &b->graph_multi))) return st;
         b->graph_flags = flags;
         b->graph_dt = dt;
         b->graph_epochs.resize(b->n);
@@ -830,8 +889,13 @@ BFB_API int bfb_batch_simulate(bfb_batch b, double dt, int n_steps, int flags) {
     } else {
         for (bfb_env e : b->envs) BFB_CUDA(cudaStreamSynchronize(e->stream));
     }
+    // each graph when a call first needs it
+    if (n_steps >= bfb_batch_s::kMultiSteps && !b->graph_multi)
+        if (int st = batch_capture(b, dt, flags, bfb_batch_s::kMultiSteps, &b->graph_multi)) return st;
+    if (n_steps % bfb_batch_s::kMultiSteps && !b->graph)
+        if (int st = batch_capture(b, dt, flags, 1, &b->graph)) return st;
     int left = n_steps;
-    for (; b->graph_multi && left >= bfb_batch_s::kMultiSteps; left -= bfb_batch_s::kMultiSteps)
+    for (; left >= bfb_batch_s::kMultiSteps; left -= bfb_batch_s::kMultiSteps)
         BFB_CUDA(cudaGraphLaunch(b->graph_multi, b->stream));
     for (; left > 0; --left) BFB_CUDA(cudaGraphLaunch(b->graph, b->stream));
     return BFB_OK;
@@ -878,7 +942,7 @@ BFB_API int bfb_batch_autotune(bfb_batch b, double dt, int flags, int trials, in
             b->warps = w;
             b->tiles_per_item = tpi;
             batch_drop_graph(b);
-            // builds both graphs and warms; then `trials` launches of the multi-step graph
+            // builds the multi-step graph and warms; then `trials` launches of it
             const int steps = trials * bfb_batch_s::kMultiSteps;
             if ((st = bfb_batch_simulate(b, dt, bfb_batch_s::kMultiSteps, flags))) break;
             cudaError_t ce = cudaEventRecord(e0, b->stream);

@@ -113,6 +113,24 @@ def test_batch_tma_items_fp64_bitexact(bfb, oracle, mode, warps, tiles):
         assert np.array_equal(env.get_field(), oracle_run(oracle, spec, dt, steps)), spec["shape"]
 
 
+@pytest.mark.parametrize("warps", [1, 2, 4])
+@pytest.mark.parametrize("steps", [3, 9])
+def test_batch_many_small_and_one_large_fp64_bitexact(bfb, oracle, warps, steps):
+    """More envs than the staged mode steps by their own kernels: small ones share stage launches
+    while one larger env (over 1 MB) runs its own chain beside them; bit for bit."""
+    dt = 0.01
+    rng = np.random.default_rng(77)
+    made = [make_instance(bfb, rng, 1, 14, 60, bfb.FP64, dt) for _ in range(39)]
+    made.append(make_instance(bfb, rng, 52, 56, 500, bfb.FP64, dt))
+    specs, envs = zip(*made)
+    batch = bfb.Batch(envs)
+    batch.set_warps(warps)
+    batch.simulate(dt, steps, bfb.STEP_DIFFUSION | bfb.STEP_CELLS)
+    batch.synchronize()
+    for spec, env in zip(specs, envs):
+        assert np.array_equal(env.get_field(), oracle_run(oracle, spec, dt, steps))
+
+
 @pytest.mark.parametrize("mode", ["staged", "persistent", "graph"])
 def test_batch_wide_substrates_fp64_bitexact(bfb, oracle, mode):
     """Envs with more than 32 substrates (a lane solves several z lines) next
