@@ -165,6 +165,7 @@ __global__ void __launch_bounds__(128, 1)
         fence_mbar_init();
     }
     __syncwarp();
+    pdl_wait();
     if (lane == 0) {
         for (int ch = 0; ch < nch; ++ch) {
             mbar_expect_tx(bar0 + 8 * ch, chunk_bytes);
@@ -250,6 +251,7 @@ __global__ void __launch_bounds__(128, 1)
             bulk_commit();
         }
     }
+    pdl_launch_dependents();
     if (lane == 0) bulk_wait_read_all();
     __syncwarp();
 }
@@ -388,6 +390,7 @@ __global__ void __launch_bounds__(128, 1) adjoint_solve_contig_pipe_kernel(Sweep
         fence_mbar_init();
     }
     __syncwarp();
+    pdl_wait();
     if (lane == 0) {
         for (int c = 0; c < nch; ++c) {
             const unsigned b = seg_bytes(c);
@@ -462,6 +465,7 @@ __global__ void __launch_bounds__(128, 1) adjoint_solve_contig_pipe_kernel(Sweep
             bulk_commit();
         }
     }
+    pdl_launch_dependents();
     if (lane == 0) bulk_wait_read_all();
     __syncwarp();
 }
@@ -505,6 +509,7 @@ __global__ void __launch_bounds__(256) adjoint_dots_kernel(const T *__restrict__
     __shared__ double s0[256 * VEC], s1[256 * VEC];
     const int S = dir.S;
     const int tid = threadIdx.x;
+    pdl_wait();
     const long long ngroups = nlines / VEC;
     const long long gidx = (long long)blockIdx.x * blockDim.x + tid;
     const long long nsegs = (long long)((n + seg - 1) / seg);
@@ -622,6 +627,107 @@ __global__ void __launch_bounds__(256) adjoint_dots_kernel(const T *__restrict__
             s0[i] += s0[i + h * S];
             s1[i] += s1[i + h * S];
         }
+        __syncthreads();
+    }
+    pdl_launch_dependents();
+    if (tid < S) {
+        double *slot = t.part + ((size_t)blockIdx.x * S + tid) * 2;
+        slot[0] += s0[tid];
+        slot[1] += s1[tid];
+    }
+}
+
+// The same sums along z where the substrates of a voxel are not whole vectors
+// (adjoint_dots_kernel would walk each line alone, two or three adjacent values
+// per warp load): the packed field is read straight through in 16-byte vectors
+// (the last elements one by one), a voxel's neighbour being the element S
+// further on, which L1 holds. Thread t takes positions VW*t + q*W, W a multiple
+// of S, so each vector lane's substrate is fixed; the block adds its lanes per
+// substrate in a fixed tree.
+// SC: the substrate count when a compile-time constant (1 to 3: part of a
+// vector's neighbours are its own elements), 0 otherwise.
+template <typename T, int VW, int SC>
+__global__ void __launch_bounds__(256) adjoint_dots_flat_kernel(const T *__restrict__ mu, const T *__restrict__ y,
+                                                                DirFaces<T> dir, long long N, int W, int steps,
+                                                                AdjTerms t) {
+    __shared__ double s0[256 * VW], s1[256 * VW];
+    const int S = SC > 0 ? SC : dir.S, nz = dir.nz, L = nz * S;
+    const int tid = threadIdx.x;
+    double dl[VW], dyy[VW];
+#pragma unroll
+    for (int u = 0; u < VW; ++u) dl[u] = dyy[u] = 0.0;
+    pdl_wait();
+    long long e0 = (long long)blockIdx.x * steps * W + VW * tid;
+#pragma unroll 2
+    for (int q = 0; q < steps; ++q, e0 += W) {
+        if (VW * tid >= W || e0 >= N) break;
+        double m0[VW], y0[VW], m1[VW], y1[VW];
+        if (e0 + VW <= N) {
+            load_vec<T, VW>(mu + e0, m0);
+            load_vec<T, VW>(y + e0, y0);
+        } else {
+#pragma unroll
+            for (int u = 0; u < VW; ++u) {
+                m0[u] = e0 + u < N ? (double)mu[e0 + u] : 0.0;
+                y0[u] = e0 + u < N ? (double)y[e0 + u] : 0.0;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < VW; ++u) {
+            if (SC > 0 && u + SC < VW) {
+                m1[u] = m0[u + SC < VW ? u + SC : u];
+                y1[u] = y0[u + SC < VW ? u + SC : u];
+            } else {
+                const long long x = min(e0 + u + S, N - 1);
+                m1[u] = (double)__ldg(mu + x);
+                y1[u] = (double)__ldg(y + x);
+            }
+        }
+        const long long row = N <= 0xffffffffLL ? (long long)((unsigned)e0 / (unsigned)L) : e0 / L;
+        const int r = (int)(e0 - row * L);
+#pragma unroll
+        for (int u = 0; u < VW; ++u) {
+            int re = r + u;  // element of its row; rows shorter than a vector may lie in between
+            long long rw = row;
+            while (re >= L) {
+                re -= L;
+                ++rw;
+            }
+            const bool first = re < S, last = re >= L - S, before = re >= L - 2 * S && !last;
+            double yu = y0[u];
+            if (dir.any && (first || last || before) && e0 + u < N) {  // y rebuilt at the ends on active z faces
+                const int d = re % S;
+                const unsigned msk = dir.mask[d];
+                if (msk & 48u) {
+                    const T *yp = y + (size_t)rw * L;
+                    const int i = (int)(rw / dir.ny), j = (int)(rw - (long long)i * dir.ny);
+                    EndFix fx;
+                    fx.make(msk & 16u, msk & 32u, nz, t.c1[d], t.c2[d], (double)dir_value(dir, i, j, 0, d),
+                            (double)dir_value(dir, i, j, nz - 1, d), nz > 1 ? (double)yp[S + d] : 0.0,
+                            nz > 1 ? (double)yp[(size_t)(nz - 2) * S + d] : 0.0);
+                    if (first && fx.lo) yu = fx.y0;
+                    if (last && fx.hi) yu = fx.yn;
+                    if (before && fx.hi) y1[u] = fx.yn;
+                }
+            }
+            if (!last) dl[u] += (m0[u] - m1[u]) * (yu - y1[u]);
+            dyy[u] += m0[u] * yu;
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < VW; ++u) {
+        s0[VW * tid + u] = dl[u];
+        s1[VW * tid + u] = dyy[u];
+    }
+    __syncthreads();
+    pdl_launch_dependents();
+    for (int p = W / S; p > 1;) {  // positions of a substrate are S apart
+        const int half = (p + 1) / 2;
+        for (int i = tid; i < (p - half) * S; i += 256) {
+            s0[i] += s0[i + half * S];
+            s1[i] += s1[i + half * S];
+        }
+        p = half;
         __syncthreads();
     }
     if (tid < S) {
@@ -781,11 +887,13 @@ __global__ void cells_keep_kernel(T *__restrict__ f, int S, int n_occ, const int
                                   T *__restrict__ vkeep) {
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= (long long)n_occ * S) return;
+    pdl_wait();
     const int s = (int)(e / S), d = (int)(e % S);
     const size_t fe = (size_t)seg_voxel[s] * S + d;
     T x = f[fe];
     vkeep[e] = x;
-    for (int q = seg_start[s]; q < seg_start[s + 1]; ++q) {
+    const int q1 = seg_start[s + 1];
+    for (int q = seg_start[s]; q < q1; ++q) {
         const size_t z = (size_t)q * S + d;
         if constexpr (sizeof(T) == 8)
             x = __ddiv_rn(__dadd_rn(x, t1[z]), t2[z]);
@@ -810,6 +918,7 @@ __global__ void cells_adjoint_kernel(T *__restrict__ lam, T *__restrict__ w, con
                                      double *__restrict__ gt2, DirFaces<T> dir) {
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= (long long)n_occ * S) return;
+    pdl_wait();
     const int s = (int)(e / S), d = (int)(e % S);
     const int vox = seg_voxel[s];
     const size_t fe = (size_t)vox * S + d;
@@ -903,7 +1012,10 @@ void opt_in_all() {
     opt_in(adjoint_strided_kernel<T>);
     opt_in(adjoint_solve_contig_pipe_kernel<T, 1>);
     opt_in(adjoint_solve_contig_pipe_kernel<T, 2>);
+    opt_in(adjoint_solve_contig_pipe_kernel<T, 3>);
     opt_in(adjoint_solve_contig_pipe_kernel<T, 4>);
+    opt_in(adjoint_solve_contig_pipe_kernel<T, 5>);
+    opt_in(adjoint_solve_contig_pipe_kernel<T, 6>);
     opt_in(adjoint_solve_contig_pipe_kernel<T, 8>);
     opt_in(adjoint_solve_contig_pipe_kernel<T, 0>);
     opt_in(adjoint_contig_kernel<T>);
@@ -960,6 +1072,27 @@ struct Adjoint {
     // 4 x 32, and ties with 4 x 128)
     static constexpr int kVec = sizeof(T) == 8 ? 2 : 4;
     static constexpr int kDotSeg = sizeof(T) == 8 ? 32 : 64;
+    static constexpr int kDotFlatBlocks = 148 * 8;  // adjoint_dots_flat_kernel, at most
+    // rows per thread: kDotSeg, fewer where that leaves under two blocks per SM
+    // (128^3 x 2 FP32: 64 blocks of 64 rows 22.6 us, 512 of 8 17.0)
+    int dots_seg(int axis) const {
+        const int n = axis_len(env, axis);
+        const long long groups = (long long)env->N / n / dots_vec(axis);
+        int seg = dots_vec(axis) == kVec ? kDotSeg : 64;
+        while (seg > 8 && groups * ((n + seg - 1) / seg) < 296LL * dots_threads()) seg /= 2;
+        return seg;
+    }
+    // z where a voxel's substrates are not whole vectors: adjoint_dots_flat_kernel, W positions a step
+    bool dots_flat(int axis) const { return axis == 2 && S % kVec != 0 && S <= 256; }
+    int dots_flat_width() const {
+        int l = S;
+        while (l % kVec) l += S;
+        return l <= kVec * 256 ? (kVec * 256) / l * l : 0;
+    }
+    int dots_flat_steps() const {  // per block
+        const long long w = dots_flat_width(), all = (env->N + w - 1) / w;
+        return (int)((all + kDotFlatBlocks - 1) / kDotFlatBlocks);
+    }
     int dots_threads() const {
         int threads = S;
         while (threads * 2 <= 256) threads *= 2;
@@ -972,7 +1105,11 @@ struct Adjoint {
     int dots_vec(int axis) const { return axis_inner(axis) % kVec == 0 ? kVec : 1; }
     long long dots_blocks(int axis) const {
         const int n = axis_len(env, axis);
-        const int sg = dots_vec(axis) == kVec ? kDotSeg : 64;
+        if (dots_flat(axis) && dots_flat_width()) {
+            const long long w = (long long)dots_flat_width() * dots_flat_steps();
+            return (env->N + w - 1) / w;
+        }
+        const int sg = dots_seg(axis);
         const long long work = (long long)env->N / n / dots_vec(axis) * ((n + sg - 1) / sg);
         return (work + dots_threads() - 1) / dots_threads();
     }
@@ -980,13 +1117,18 @@ struct Adjoint {
         const int n = axis_len(env, axis);
         const long long nlines = (long long)env->N / n;
         const unsigned blocks = (unsigned)dots_blocks(axis);
-        if (dots_vec(axis) == kVec)
-            adjoint_dots_kernel<T, kVec><<<blocks, dots_threads(), 0, st>>>(mu, y, a.dir, axis, n, axis_inner(axis),
-                                                                             nlines, kDotSeg, t);
-        else
-            adjoint_dots_kernel<T, 1><<<blocks, dots_threads(), 0, st>>>(mu, y, a.dir, axis, n, axis_inner(axis),
-                                                                          nlines, 64, t);
-        BFB_CUDA(cudaGetLastError());
+        const int seg = dots_seg(axis);
+        if (dots_flat(axis) && dots_flat_width()) {
+            const auto k = S == 1   ? adjoint_dots_flat_kernel<T, kVec, 1>
+                           : S == 2 ? adjoint_dots_flat_kernel<T, kVec, 2>
+                           : S == 3 ? adjoint_dots_flat_kernel<T, kVec, 3>
+                                    : adjoint_dots_flat_kernel<T, kVec, 0>;
+            BFB_CUDA(launch_pdl(k, blocks, 256, 0, st, mu, y, a.dir, (long long)env->N,
+                                dots_flat_width(), dots_flat_steps(), t));
+        } else {
+            const auto k = dots_vec(axis) == kVec ? adjoint_dots_kernel<T, kVec> : adjoint_dots_kernel<T, 1>;
+            BFB_CUDA(launch_pdl(k, blocks, dots_threads(), 0, st, mu, y, a.dir, axis, n, axis_inner(axis), nlines, seg, t));
+        }
         return BFB_OK;
     }
 
@@ -1004,8 +1146,8 @@ struct Adjoint {
                 const int crow = lam.crow[axis];
                 const size_t wb = strided_tma_warp_bytes(g.n, crow, sizeof(T), 32);
                 if (wb <= (size_t)kMaxSmem) {
-                    adjoint_solve_strided_tma_kernel<T><<<tiles, 32, wb, st>>>(lam.map[axis], mu.map[axis], a, g, crow);
-                    BFB_CUDA(cudaGetLastError());
+                    BFB_CUDA(launch_pdl(adjoint_solve_strided_tma_kernel<T>, tiles, 32, wb, st, lam.map[axis],
+                                        mu.map[axis], a, g, crow));
                     return sums ? dots(axis, a, static_cast<const T *>(mu.p), yp, t) : BFB_OK;
                 }
             }
@@ -1018,14 +1160,18 @@ struct Adjoint {
         const unsigned tiles = (unsigned)tiles_z;
         if (kc > 0) {
             const size_t wb = (128 + (size_t)gz.R * gz.RS * sizeof(T) + 127) / 128 * 128;
+            auto k = adjoint_solve_contig_pipe_kernel<T, 0>;
             switch (S) {
-            case 1: adjoint_solve_contig_pipe_kernel<T, 1><<<tiles, 32, wb, st>>>(a, gz, kc); break;
-            case 2: adjoint_solve_contig_pipe_kernel<T, 2><<<tiles, 32, wb, st>>>(a, gz, kc); break;
-            case 4: adjoint_solve_contig_pipe_kernel<T, 4><<<tiles, 32, wb, st>>>(a, gz, kc); break;
-            case 8: adjoint_solve_contig_pipe_kernel<T, 8><<<tiles, 32, wb, st>>>(a, gz, kc); break;
-            default: adjoint_solve_contig_pipe_kernel<T, 0><<<tiles, 32, wb, st>>>(a, gz, kc); break;
+            case 1: k = adjoint_solve_contig_pipe_kernel<T, 1>; break;
+            case 2: k = adjoint_solve_contig_pipe_kernel<T, 2>; break;
+            case 3: k = adjoint_solve_contig_pipe_kernel<T, 3>; break;
+            case 4: k = adjoint_solve_contig_pipe_kernel<T, 4>; break;
+            case 5: k = adjoint_solve_contig_pipe_kernel<T, 5>; break;
+            case 6: k = adjoint_solve_contig_pipe_kernel<T, 6>; break;
+            case 8: k = adjoint_solve_contig_pipe_kernel<T, 8>; break;
+            default: break;
             }
-            BFB_CUDA(cudaGetLastError());
+            BFB_CUDA(launch_pdl(k, tiles, 32, wb, st, a, gz, kc));
             return sums ? dots(2, a, static_cast<const T *>(mu.p), yp, t) : BFB_OK;
         }
         const size_t smem = 2 * (size_t)gz.R * gz.RS * sizeof(T);
@@ -1055,10 +1201,18 @@ int adjoint_run(bfb_env_s *env, double dt, int n_steps, int flags, int K, const 
     if ((rc = env_tile_plan(env, sizeof(T), env->nz * S, &A.gx, &A.gy, &A.gz, vb16))) return rc;
     opt_in_all<T>();
     const long long tiles_x = (long long)A.gx.n_slabs * A.gx.ncb, tiles_y = (long long)A.gy.n_slabs * A.gy.ncb;
-    A.tiles_z = (A.gz.nrows + A.gz.R - 1) / A.gz.R;
     {   // pipelined z solve: the forward pipe kernel's alignment rules
         const long long L = (long long)env->nz * S;
         const int eb = (int)sizeof(T);
+        // 16-byte shared rows where the conflict-free stride is not (as the
+        // forward z sweep; 128^3 x 2 FP32: the kernel without bulk copies took
+        // 57 us with its sums, this one 18.5 and the sums 33)
+        if (env->use_tma && S <= 32 && (L * eb) % 16 == 0 && ((long long)A.gz.RS * eb) % 16 != 0) {
+            ContigGeom gt = A.gz;
+            if (contig_aligned_geom(env->nz, S, (int)L, eb, &gt.R, &gt.RS) &&
+                128 + (size_t)gt.R * gt.RS * eb + 127 <= (size_t)kMaxSmem)
+                A.gz = gt;
+        }
         const size_t wb = (128 + (size_t)A.gz.R * A.gz.RS * eb + 127) / 128 * 128;
         if (env->use_tma && S <= 32 && (L * eb) % 16 == 0 && ((long long)A.gz.RS * eb) % 16 == 0 &&
             wb <= (size_t)kMaxSmem) {
@@ -1068,6 +1222,7 @@ int adjoint_run(bfb_env_s *env, double dt, int n_steps, int flags, int K, const 
             A.kc = (kc + q - 1) / q * q;
         }
     }
+    A.tiles_z = (A.gz.nrows + A.gz.R - 1) / A.gz.R;
 
     // ---- workspace
     const int nseg = (n_steps + K - 1) / K;
@@ -1165,10 +1320,8 @@ int adjoint_run(bfb_env_s *env, double dt, int n_steps, int flags, int K, const 
                 (r = A.fwd(2, S2[j], W[j])))
                 return r;
             if (cells) {
-                cells_keep_kernel<T><<<occ_blocks, 256, 0, st>>>(static_cast<T *>(W[j].p), S, env->n_occ,
-                                                                 env->seg_start, env->seg_voxel, t1, t2,
-                                                                 vkeep + (size_t)j * occ);
-                BFB_CUDA(cudaGetLastError());
+                BFB_CUDA(launch_pdl(cells_keep_kernel<T>, occ_blocks, 256, 0, st, static_cast<T *>(W[j].p), S, env->n_occ,
+                                    env->seg_start, env->seg_voxel, t1, t2, vkeep + (size_t)j * occ));
             }
         }
         return BFB_OK;
@@ -1218,10 +1371,9 @@ int adjoint_run(bfb_env_s *env, double dt, int n_steps, int flags, int K, const 
             if (cells) {
                 DirFaces<T> dj = dirf;
                 if (s == nseg - 1 && j == len - 1) dj.any = 0;  // dL/d(final field) is not masked
-                cells_adjoint_kernel<T><<<occ_blocks, 256, 0, st>>>(
-                    static_cast<T *>(pl->p), static_cast<T *>(W[j].p), vkeep + (size_t)j * occ, S, env->n_occ,
-                    env->seg_start, env->seg_voxel, t1, t2, gt1, gt2, dj);
-                BFB_CUDA(cudaGetLastError());
+                BFB_CUDA(launch_pdl(cells_adjoint_kernel<T>, occ_blocks, 256, 0, st, static_cast<T *>(pl->p),
+                                    static_cast<T *>(W[j].p), vkeep + (size_t)j * occ, S, env->n_occ, env->seg_start,
+                                    env->seg_voxel, t1, t2, gt1, gt2, dj));
             }
             if ((rc = A.adj(2, *pl, W[j], *pm))) return rc;
             if ((rc = A.adj(1, *pm, S2[j], *pl))) return rc;

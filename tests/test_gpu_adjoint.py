@@ -112,6 +112,23 @@ def test_adjoint_fp64_matches_oracle(bfb, oracle, n_steps, K, shape, S, agents):
     env.close()
 
 
+@pytest.mark.parametrize("shape,S", [((3, 2, 2), 1), ((5, 4, 2), 3), ((6, 3, 4), 1), ((4, 5, 16), 3), ((9, 7, 34), 5),
+                                     ((40, 33, 4), 7)])
+def test_adjoint_z_sums_of_odd_substrate_counts(bfb, oracle, shape, S):
+    """Rows of whole 16-byte vectors whose substrates are not: the z solve on aligned shared rows
+    and the z sums read straight through the field, with lines of two rows, vectors across voxels
+    and rows, the last vector and faces at both ends."""
+    rng = np.random.default_rng(900 + S + shape[2])
+    dt = 0.01
+    env, D, lam, rho0, dirv, ag = _setup(bfb, bfb.FP64, shape, S, rng, dt=dt)
+    w = rng.standard_normal(rho0.shape)
+    ref = oracle_adjoint(oracle, rho0, w, 3, dt, env.dx, D, lam, dirv, ag)
+    got = _gpu_adjoint(bfb, env, rho0, w, 3, dt, 2, ag)
+    for k in ("initial", "D", "lambda"):
+        assert _rel(got[k], ref[k]) <= 1e-11, k
+    env.close()
+
+
 def test_adjoint_is_deterministic(bfb):
     rng = np.random.default_rng(9)
     env, D, lam, rho0, dirv, ag = _setup(bfb, bfb.FP64, (40, 36, 44), 3, rng, n_agents=300)
