@@ -889,8 +889,9 @@ BFB_API int bfb_batch_simulate(bfb_batch b, double dt, int n_steps, int flags) {
     } else {
         for (bfb_env e : b->envs) BFB_CUDA(cudaStreamSynchronize(e->stream));
     }
-    // each graph when a call first needs it
-    if (n_steps >= bfb_batch_s::kMultiSteps && !b->graph_multi)
+    // the eight-step graph at once (a first short call warms later long ones),
+    // the one-step graph when a call has a remainder
+    if (n_steps > 0 && !b->graph_multi)
         if (int st = batch_capture(b, dt, flags, bfb_batch_s::kMultiSteps, &b->graph_multi)) return st;
     if (n_steps % bfb_batch_s::kMultiSteps && !b->graph)
         if (int st = batch_capture(b, dt, flags, 1, &b->graph)) return st;

@@ -949,6 +949,8 @@ BFB_API int bfb_simulate(bfb_env env, double dt, int n_steps, int flags) {
     if (n_steps == 0) return BFB_OK;
     NvtxRange range("bfb_simulate");
     if (!env->use_graphs || env->stream == nullptr) return run_steps_any(env, dt, n_steps, flags, env->stream);
+    if (env->stream == cudaStreamLegacy)  // cannot be captured, now or later
+        return cuda_fail(cudaErrorStreamCaptureUnsupported, "bfb_simulate on the legacy stream (BFB_OPT_USE_GRAPHS is on)");
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     BFB_CUDA(cudaStreamIsCapturing(env->stream, &capturing));
     if (capturing != cudaStreamCaptureStatusNone)  // a graph launch cannot be captured
