@@ -15,6 +15,8 @@
 // warp fits the class. Each group of envs (about equal work) runs its chain of
 // stage launches on its own stream, forked from and joined to the batch stream
 // inside the graph; stream order alone orders the stages, so no warp waits.
+// Larger envs, and all envs of a small batch, are stepped by their own kernels
+// on chains beside those (kOwnChainBytes).
 //
 // Persistent: one launch of batch_step_kernel per step, a grid of resident
 // CTAs whose warps pull work items from a device queue (one atomic counter).

@@ -61,7 +61,7 @@ typedef struct bfb_env_s *bfb_env;
 #define BFB_OPT_FREEZE_FACTORS 1 /* 1 (default): Thomas factors are computed on the first step
                                     and kept, as BioFVM_parallel.cpp:714,913 does; 0: recomputed
                                     whenever dt differs from the cached one */
-#define BFB_OPT_USE_GRAPHS 2     /* 1 (default): bfb_simulate replays a captured CUDA graph */
+#define BFB_OPT_USE_GRAPHS 2     /* 1 (default): bfb_simulate replays a captured CUDA graph once the same steps keep coming */
 #define BFB_OPT_USE_TMA 3        /* 1 (default): sweeps move data with the TMA engine where the
                                     grid's row pitch allows; 0: cp.async kernels everywhere */
 
@@ -268,7 +268,9 @@ BFB_API int bfb_checksum(bfb_env env, double *out);
  * every env -- and, with BFB_STEP_CELLS, its agents -- replayed from a CUDA
  * graph, in one of three modes:
  *   BFB_BATCH_MODE_STAGED (default): one launch per stage (x, y, z sweeps,
- *     agents), each a flat grid over every env's tiles, one warp per tile;
+ *     agents), each a flat grid over the envs' tiles, one warp per tile;
+ *     larger envs, and all envs of a small batch, are stepped by their own
+ *     kernels beside them;
  *   BFB_BATCH_MODE_PERSISTENT: ONE persistent kernel launch per step whose
  *     warps pull (env, stage, tile) work items from a device queue;
  *   BFB_BATCH_MODE_GRAPH: every env's own step kernels (as bfb_simulate
