@@ -32,13 +32,18 @@ def _run(cmd):
     subprocess.run([str(c) for c in cmd], check=True)
 
 
+def dependencies() -> list[Path]:
+    """Every file the libraries are compiled from: a change to one rebuilds them."""
+    return ([p for p in sorted(CSRC.iterdir()) if p.suffix in (".cu", ".cuh", ".h")] +
+            [ROOT / "include" / "biofvm_b200.h"] +
+            list((PKG / "host").rglob("*.cpp")) + list((PKG / "host").glob("*.h")))
+
+
 def build(force: bool = False, verbose_ptxas: bool = False) -> Path:
     LIB_DIR.mkdir(exist_ok=True)
     obj_dir = PKG / "_build"
     obj_dir.mkdir(exist_ok=True)
-    deps = ([CSRC / s for s in SOURCES] + list(CSRC.glob("*.cuh")) + [ROOT / "include" / "biofvm_b200.h"] +
-            list((PKG / "host").rglob("*.cpp")) + list((PKG / "host").glob("*.h")))
-    newest = max(p.stat().st_mtime for p in deps)
+    newest = max(p.stat().st_mtime for p in dependencies())
     if LIB.exists() and LIB.stat().st_mtime >= newest and not force:
         return LIB
     extra = ["-Xptxas", "-v"] if verbose_ptxas else []

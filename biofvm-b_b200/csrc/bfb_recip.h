@@ -21,6 +21,7 @@
 #pragma once
 #include <cmath>
 #include <cstdint>
+#include <initializer_list>
 
 namespace bfb {
 
