@@ -27,23 +27,24 @@ namespace bfb {
 
 constexpr int kRecipWindow = 16;
 
-// Calls f(X) for every candidate numerator of divisor mantissa Y; stops when f returns false.
-template <typename F>
+// Calls f(X) for every candidate numerator of divisor mantissa Y (P-bit
+// mantissas, residues up to W); stops when f returns false.
+template <int P = 53, int W = kRecipWindow, typename F>
 inline bool recip_candidates(uint64_t Y, F f) {
-    constexpr uint64_t lo = 1ull << 52, hi = 1ull << 53;
+    constexpr uint64_t lo = 1ull << (P - 1), hi = 1ull << P;
     int s = 0;  // Y = 2^s Yo: X 2^k = r (mod Y) needs 2^s | r, and then X = r 2^-k (mod Yo)
     uint64_t Yo = Y;
     while (!(Yo & 1)) {
         Yo >>= 1;
         ++s;
     }
-    if (s > 4) return true;  // every |r| <= 16 but 0 is ruled out (and for Yo = 1 the reciprocal is exact)
+    if ((W >> s) == 0) return true;  // every |r| <= W but 0 is ruled out (and for Yo = 1 the reciprocal is exact)
     uint64_t inv = 1;  // 2^-k mod Yo
-    for (int k = 1; k <= 54; ++k) {
+    for (int k = 1; k <= P + 1; ++k) {
         inv = (inv & 1) ? (inv + Yo) >> 1 : inv >> 1;
-        if (k < 53) continue;
+        if (k < P) continue;
         uint64_t x = 0;
-        for (int r = 1; r <= kRecipWindow; ++r) {
+        for (int r = 1; r <= W; ++r) {
             x += inv;  // r 2^-k mod Yo
             if (x >= Yo) x -= Yo;
             if (s && (r & ((1 << s) - 1))) continue;
@@ -51,7 +52,7 @@ inline bool recip_candidates(uint64_t Y, F f) {
                 uint64_t X = sign ? Yo - x : x;
                 if (X < lo) X += (lo - X + Yo - 1) / Yo * Yo;
                 for (; X < hi; X += Yo)
-                    if ((k == 53) == (X >= Y) && !f(X)) return false;
+                    if ((k == P) == (X >= Y) && !f(X)) return false;
             }
         }
     }
