@@ -50,6 +50,7 @@
 #include "bfb_aux.cuh"
 #include "bfb_tiles.cuh"
 #include "bfb_tma.cuh"
+#include "bfb_upload.h"
 
 namespace bfb {
 
@@ -1303,7 +1304,8 @@ int adjoint_run(bfb_env_s *env, double dt, int n_steps, int flags, int K, const 
         hcoef[S + d] = c2;
     }
     A.coef = coef;
-    BFB_CUDA(cudaMemcpyAsync(coef, hcoef.data(), sizeof(double) * 2 * S, cudaMemcpyHostToDevice, st));
+    Uploads up(st);
+    BFB_CUDA(up.copy(coef, std::move(hcoef)));
     BFB_CUDA(cudaMemsetAsync(part, 0, sizeof(double) * 2 * S * slots, st));
     if (nact) {
         BFB_CUDA(cudaMemsetAsync(gt1, 0, sizeof(double) * nact, st));
@@ -1403,7 +1405,7 @@ int adjoint_run(bfb_env_s *env, double dt, int n_steps, int flags, int K, const 
             (env->dx * env->dx) * env->dx, grates, grates + nlist, grates + 2 * nlist);
         BFB_CUDA(cudaGetLastError());
     }
-    BFB_CUDA(cudaStreamSynchronize(st));
+    BFB_CUDA(up.wait());
     int herr = 0;
     BFB_CUDA(cudaMemcpy(&herr, env->d_err, sizeof(int), cudaMemcpyDeviceToHost));
     if (herr) return fail(BFB_ERR_WATCHDOG, "adjoint: a device-side wait ran out of its iteration limit");

@@ -7,6 +7,8 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "bfb_upload.h"
+
 namespace bfb {
 
 // ---------------------------------------------------------------------------
@@ -290,10 +292,10 @@ int agents_sort(bfb_env_s *env, int n, AgentScratch &w) {
 }
 
 // Waits for the build and takes the counts the launches are sized by.
-int agents_finish(bfb_env_s *env, const AgentScratch &w) {
+int agents_finish(bfb_env_s *env, Uploads &up, const AgentScratch &w) {
     int counts[2] = {0, 0};
     BFB_CUDA(cudaMemcpyAsync(counts, w.counts, sizeof(counts), cudaMemcpyDeviceToHost, env->stream));
-    BFB_CUDA(cudaStreamSynchronize(env->stream));
+    BFB_CUDA(up.wait());
     env->n_occ = counts[0];
     env->n_active = counts[1];
     return BFB_OK;
@@ -319,8 +321,9 @@ int agents_build(bfb_env_s *env, int n, const double *pos, const double *volume,
     cudaStream_t s = env->stream;
     AgentScratch w;
     if ((st = agents_layout(env, n, true, &w))) return st;
-    BFB_CUDA(cudaMemcpyAsync(w.pos, pos, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, s));
-    if (active) BFB_CUDA(cudaMemcpyAsync(w.active, active, n, cudaMemcpyHostToDevice, s));
+    Uploads up(s);  // the caller's arrays: no return before their copies are done
+    BFB_CUDA(up.copy(w.pos, pos, sizeof(double) * 3 * n));
+    if (active) BFB_CUDA(up.copy(w.active, active, n));
     BinGeom g;
     for (int a = 0; a < 3; ++a) {
         g.lo[a] = env->bbox[a];
@@ -335,10 +338,10 @@ int agents_build(bfb_env_s *env, int n, const double *pos, const double *volume,
     env->n_agents = n;
     if ((st = agents_sort(env, n, w))) return st;
     // the rates cross the host link while the sort runs
-    BFB_CUDA(cudaMemcpyAsync(env->ag_vol, volume, sizeof(double) * n, cudaMemcpyHostToDevice, s));
-    BFB_CUDA(cudaMemcpyAsync(env->ag_sec, sec, sizeof(double) * nS, cudaMemcpyHostToDevice, s));
-    BFB_CUDA(cudaMemcpyAsync(env->ag_upt, upt, sizeof(double) * nS, cudaMemcpyHostToDevice, s));
-    BFB_CUDA(cudaMemcpyAsync(env->ag_sat, sat, sizeof(double) * nS, cudaMemcpyHostToDevice, s));
+    BFB_CUDA(up.copy(env->ag_vol, volume, sizeof(double) * n));
+    BFB_CUDA(up.copy(env->ag_sec, sec, sizeof(double) * nS));
+    BFB_CUDA(up.copy(env->ag_upt, upt, sizeof(double) * nS));
+    BFB_CUDA(up.copy(env->ag_sat, sat, sizeof(double) * nS));
     const unsigned gb = (unsigned)((nS + 255) / 256);
     if (env->precision == BFB_FP64)
         agent_constants_kernel<double><<<gb, 256, 0, s>>>(w.counts, S, env->ag_order, env->ag_vol, env->ag_sec,
@@ -349,7 +352,7 @@ int agents_build(bfb_env_s *env, int n, const double *pos, const double *volume,
                                                          env->ag_upt, env->ag_sat, dt, g.dV, (float *)env->ag_t1,
                                                          (float *)env->ag_t2);
     BFB_CUDA(cudaGetLastError());
-    if ((st = agents_finish(env, w))) return st;
+    if ((st = agents_finish(env, up, w))) return st;
     env->rates_known = true;
     return BFB_OK;
 }
@@ -363,20 +366,19 @@ int agents_build_constants(bfb_env_s *env, int n, const int *voxel, const double
     cudaStream_t s = env->stream;
     AgentScratch w;
     if ((st = agents_layout(env, n, false, &w))) return st;
-    BFB_CUDA(cudaMemcpyAsync(env->agent_voxel, voxel, sizeof(int) * n, cudaMemcpyHostToDevice, s));
+    Uploads up(s);
+    BFB_CUDA(up.copy(env->agent_voxel, voxel, sizeof(int) * n));
     env->n_agents = n;
     for (int a = 0; a < n; ++a)
-        if ((!active || active[a]) && (voxel[a] < 0 || voxel[a] >= env->V)) {
-            BFB_CUDA(cudaStreamSynchronize(s));
+        if ((!active || active[a]) && (voxel[a] < 0 || voxel[a] >= env->V))
             return fail(BFB_ERR_INVALID_ARG, "agent voxel index out of range");
-        }
-    if (active) BFB_CUDA(cudaMemcpyAsync(w.active, active, n, cudaMemcpyHostToDevice, s));
+    if (active) BFB_CUDA(up.copy(w.active, active, n));
     key_agents_kernel<<<(n + 127) / 128, 128, 0, s>>>(n, env->agent_voxel, active ? w.active : nullptr, (int)env->V,
                                                       w.key, w.idx);
     BFB_CUDA(cudaGetLastError());
     if ((st = agents_sort(env, n, w))) return st;
-    BFB_CUDA(cudaMemcpyAsync(w.t1, t1, sizeof(double) * nS, cudaMemcpyHostToDevice, s));
-    BFB_CUDA(cudaMemcpyAsync(w.t2, t2, sizeof(double) * nS, cudaMemcpyHostToDevice, s));
+    BFB_CUDA(up.copy(w.t1, t1, sizeof(double) * nS));
+    BFB_CUDA(up.copy(w.t2, t2, sizeof(double) * nS));
     const unsigned gb = (unsigned)((nS + 255) / 256);
     if (env->precision == BFB_FP64)
         gather_constants_kernel<double><<<gb, 256, 0, s>>>(w.counts, S, env->ag_order, w.t1, w.t2,
@@ -385,7 +387,7 @@ int agents_build_constants(bfb_env_s *env, int n, const int *voxel, const double
         gather_constants_kernel<float><<<gb, 256, 0, s>>>(w.counts, S, env->ag_order, w.t1, w.t2, (float *)env->ag_t1,
                                                           (float *)env->ag_t2);
     BFB_CUDA(cudaGetLastError());
-    return agents_finish(env, w);
+    return agents_finish(env, up, w);
 }
 
 int launch_cells(bfb_env_s *env, cudaStream_t s) {

@@ -39,6 +39,7 @@
 #include "bfb_aux.cuh"
 #include "bfb_tiles.cuh"
 #include "bfb_tma_tiles.cuh"
+#include "bfb_upload.h"
 
 namespace bfb {
 
@@ -566,11 +567,6 @@ static int batch_upload(bfb_batch_s *b, double dt) {
             b->stage_base[s + 1][f] = b->stage_base[s][f] + cnt;
         }
     }
-    BFB_CUDA(cudaMemcpyAsync(b->d_maps, maps.data(), sizeof(CUtensorMap) * maps.size(), cudaMemcpyHostToDevice, b->stream));
-    BFB_CUDA(cudaMemcpyAsync(b->d_inst, inst.data(), sizeof(BatchInst<T>) * b->n, cudaMemcpyHostToDevice, b->stream));
-    BFB_CUDA(cudaMemcpyAsync(b->d_prefix, prefix.data(), sizeof(int) * prefix.size(), cudaMemcpyHostToDevice, b->stream));
-    BFB_CUDA(cudaMemcpyAsync(b->d_tpre, tpre.data(), sizeof(int) * tpre.size(), cudaMemcpyHostToDevice, b->stream));
-    BFB_CUDA(cudaMemcpyAsync(b->d_perm, perm.data(), sizeof(int) * perm.size(), cudaMemcpyHostToDevice, b->stream));
     b->tma_only = true;
     for (int k = 0; k < b->n; ++k) b->tma_only = b->tma_only && inst[k].tma[0] && inst[k].tma[1] && inst[k].tma[2];
     const void *step_kernel = b->tma_only ? (const void *)batch_step_kernel<T, true>
@@ -595,6 +591,13 @@ static int batch_upload(bfb_batch_s *b, double dt) {
         BFB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, step_kernel, 32 * w, bytes));
         b->grid[w] = per_sm * sms;
     }
+    Uploads up(b->stream);
+    BFB_CUDA(up.copy(b->d_maps, std::move(maps)));
+    BFB_CUDA(up.copy(b->d_inst, std::move(inst)));
+    BFB_CUDA(up.copy(b->d_prefix, std::move(prefix)));
+    BFB_CUDA(up.copy(b->d_tpre, std::move(tpre)));
+    BFB_CUDA(up.copy(b->d_perm, std::move(perm)));
+    BFB_CUDA(up.wait());
     return BFB_OK;
 }
 

@@ -12,6 +12,7 @@
 #include "bfb_internal.cuh"
 #include "bfb_recip.h"
 #include "bfb_sweeps.cuh"
+#include "bfb_upload.h"
 
 namespace bfb {
 
@@ -70,35 +71,33 @@ static void axis_factors(int n, int S, double dt, double dx, const double *D, co
     }
 }
 
-// Uploads go through the env's stream and their callers wait for it: a copy
-// from pageable memory on the legacy stream may return before its last bytes
-// are on the device, and kernels on the env's non-blocking stream do not wait
-// for that stream.
-static int upload_table(bfb_env_s *env, void *dst, const std::vector<double> &v) {
+// Uploads go through the env's stream and their callers wait for it (Uploads):
+// a copy from pageable memory on the legacy stream may return before its last
+// bytes are on the device, and kernels on the env's non-blocking stream do not
+// wait for that stream.
+static int upload_table(bfb_env_s *env, Uploads &up, void *dst, std::vector<double> v) {
     if (env->precision == BFB_FP64) {
-        BFB_CUDA(cudaMemcpyAsync(dst, v.data(), v.size() * sizeof(double), cudaMemcpyHostToDevice, env->stream));
+        BFB_CUDA(up.copy(dst, std::move(v)));
     } else {
         std::vector<float> f(v.size());
         for (size_t q = 0; q < v.size(); ++q) f[q] = (float)v[q];
-        BFB_CUDA(cudaMemcpyAsync(dst, f.data(), f.size() * sizeof(float), cudaMemcpyHostToDevice, env->stream));
+        BFB_CUDA(up.copy(dst, std::move(f)));
     }
     return BFB_OK;
 }
 
 // A packed V*S host table (the reference layout) into a device array laid
 // out like the field (rows at the pitch Lp), in the env's precision.
-static int upload_pitched_table(bfb_env_s *env, void *dst, const std::vector<double> &v) {
+static int upload_pitched_table(bfb_env_s *env, Uploads &up, void *dst, std::vector<double> v) {
     const size_t rows = (size_t)env->nx * env->ny, L = (size_t)env->nz * env->S;
     const size_t eb = env->elem;
-    std::vector<float> f;
-    const void *src = v.data();
     if (env->precision == BFB_FP32) {
-        f.resize(v.size());
+        std::vector<float> f(v.size());
         for (size_t q = 0; q < v.size(); ++q) f[q] = (float)v[q];
-        src = f.data();
+        BFB_CUDA(up.copy_rows(dst, (size_t)env->Lp * eb, std::move(f), L * eb, rows));
+    } else {
+        BFB_CUDA(up.copy_rows(dst, (size_t)env->Lp * eb, std::move(v), L * eb, rows));
     }
-    BFB_CUDA(cudaMemcpy2DAsync(dst, (size_t)env->Lp * eb, src, L * eb, L * eb, rows, cudaMemcpyHostToDevice,
-                               env->stream));
     return BFB_OK;
 }
 
@@ -123,7 +122,7 @@ static int tail_start(const std::vector<std::vector<double>> &tabs, int n, int S
 //         are proven.
 //   FP32: 1/den as a hi+lo pair of floats, c1/den and c rounded once; the
 //         deviation form of the FP32 kernels (bfb_sweeps.cuh) needs no c1.
-static int upload_factors(bfb_env_s *env, int axis, int n, const std::vector<double> &den,
+static int upload_factors(bfb_env_s *env, Uploads &up, int axis, int n, const std::vector<double> &den,
                           const std::vector<double> &c, const std::vector<double> &c1) {
     const int S = env->S;
     const size_t nS = (size_t)n * S;
@@ -174,11 +173,11 @@ static int upload_factors(bfb_env_s *env, int axis, int n, const std::vector<dou
     for (size_t k = 0; k < tabs.size(); ++k)
         for (int d = 0; d < S; ++d)
             for (int m = 0; m < std::min(hpad, n); ++m) head[(k * S + d) * hpad + m] = tabs[k][(size_t)m * S + d];
-    int st = upload_table(env, env->fac_tab[axis], flat);
+    int st = upload_table(env, up, env->fac_tab[axis], std::move(flat));
     if (st) return st;
-    st = upload_table(env, env->fac_tail[axis], tail);
+    st = upload_table(env, up, env->fac_tail[axis], std::move(tail));
     if (st) return st;
-    st = upload_table(env, env->fac_head[axis], head);
+    st = upload_table(env, up, env->fac_head[axis], std::move(head));
     if (st) return st;
     env->fac_m0[axis] = m0;
     env->fac_fast[axis] = fast;
@@ -192,12 +191,13 @@ static int ensure_factors(bfb_env_s *env, double dt) {
     std::vector<double> den, c, c1;
     // the factor tables are only read by kernels on env->stream
     BFB_CUDA(cudaStreamSynchronize(env->stream));
+    Uploads up(env->stream);
     for (int a = 0; a < 3; ++a) {
         axis_factors(ns[a], env->S, dt, env->dx, env->D.data(), env->lambda.data(), den, c, c1);
-        int st = upload_factors(env, a, ns[a], den, c, c1);
+        int st = upload_factors(env, up, a, ns[a], den, c, c1);
         if (st) return st;
     }
-    int st = upload_table(env, env->c1, c1);
+    int st = upload_table(env, up, env->c1, std::move(c1));
     if (st) return st;
     // g = 1/(1 + c2), c2 = dt*lambda/3 (BioFVM_parallel.cpp:793-794), as hi, lo
     std::vector<double> g(2 * (size_t)env->S);
@@ -208,8 +208,8 @@ static int ensure_factors(bfb_env_s *env, double dt) {
         g[d] = (double)(float)gv;
         g[env->S + d] = (double)(float)(gv - g[d]);
     }
-    if ((st = upload_table(env, env->g, g))) return st;
-    BFB_CUDA(cudaStreamSynchronize(env->stream));
+    if ((st = upload_table(env, up, env->g, std::move(g)))) return st;
+    BFB_CUDA(up.wait());
     env->factors_valid = true;
     env->factor_dt = dt;
     env->epoch++;
@@ -405,10 +405,11 @@ static int bulk_tabulate(bfb_env_s *env, const double *Sr, const double *T, cons
         BFB_CUDA(cudaMemsetAsync(env->bulkB, 0, env->elem * env->Np, env->stream));
     }
     BFB_CUDA(cudaStreamSynchronize(env->stream));
-    int st = upload_pitched_table(env, env->bulkA, A);
-    if (!st) st = upload_pitched_table(env, env->bulkB, B);
+    Uploads up(env->stream);
+    int st = upload_pitched_table(env, up, env->bulkA, std::move(A));
+    if (!st) st = upload_pitched_table(env, up, env->bulkB, std::move(B));
     if (st) return st;
-    BFB_CUDA(cudaStreamSynchronize(env->stream));
+    BFB_CUDA(up.wait());
     return BFB_OK;
 }
 
@@ -763,7 +764,7 @@ BFB_API int bfb_field_pitch(bfb_env env, int *row_elems) {
 }
 
 // Dirichlet: cut the six face arrays out of per-voxel values.
-static int dirichlet_install(bfb_env_s *env, const std::vector<double> *faces_host /* 6 arrays or null */,
+static int dirichlet_install(bfb_env_s *env, std::vector<double> *faces_host /* 6 arrays (taken) or null */,
                              const uint8_t *activation, const uint8_t *face_mask) {
     const int S = env->S;
     if (activation) env->activation.assign(activation, activation + S);
@@ -790,13 +791,14 @@ static int dirichlet_install(bfb_env_s *env, const std::vector<double> *faces_ho
             BFB_CUDA(cudaMemsetAsync(env->faces[f], 0, env->elem * fsz[f] * S, env->stream));
         }
     BFB_CUDA(cudaStreamSynchronize(env->stream));
+    Uploads up(env->stream);
     if (faces_host)
         for (int f = 0; f < 6; ++f) {
-            int st = upload_table(env, env->faces[f], faces_host[f]);
+            int st = upload_table(env, up, env->faces[f], std::move(faces_host[f]));
             if (st) return st;
         }
-    BFB_CUDA(cudaMemcpyAsync(env->d_mask, bits.data(), S, cudaMemcpyHostToDevice, env->stream));
-    BFB_CUDA(cudaStreamSynchronize(env->stream));
+    BFB_CUDA(up.copy(env->d_mask, std::move(bits)));
+    BFB_CUDA(up.wait());
     env->dir_any = any != 0;
     env->epoch++;
     return BFB_OK;
