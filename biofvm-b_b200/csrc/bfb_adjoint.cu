@@ -382,8 +382,8 @@ __global__ void __launch_bounds__(128, 1) adjoint_solve_contig_pipe_kernel(Sweep
     unsigned char *wbase = smem_raw + (size_t)warp * wbytes;
     const unsigned bar0 = smem_u32(wbase);
     T *__restrict__ sm = reinterpret_cast<T *>(wbase + 128);
-    const T *__restrict__ base = a.f + (size_t)row0 * L;
-    T *__restrict__ obase = a.fo + (size_t)row0 * L;
+    const T *base = a.f + (size_t)row0 * L;
+    T *obase = a.fo + (size_t)row0 * L;
     auto seg_bytes = [&](int c) -> unsigned { return (unsigned)((min(nz, (c + 1) * kc) - c * kc) * S * (int)sizeof(T)); };
 
     if (lane == 0) {
@@ -504,9 +504,9 @@ __device__ __forceinline__ void load_vec(const T *p, double (&o)[VEC]) {
 }
 
 template <typename T, int VEC>
-__global__ void __launch_bounds__(256) adjoint_dots_kernel(const T *__restrict__ mu, const T *__restrict__ y,
-                                                           DirFaces<T> dir, int axis, int n, long long inner,
-                                                           long long nlines, int seg, AdjTerms t) {
+__global__ void __launch_bounds__(256) adjoint_dots_kernel(const T *mu, const T *y, DirFaces<T> dir, int axis,
+                                                           int n, long long inner, long long nlines, int seg,
+                                                           AdjTerms t) {
     __shared__ double s0[256 * VEC], s1[256 * VEC];
     const int S = dir.S;
     const int tid = threadIdx.x;
@@ -523,8 +523,8 @@ __global__ void __launch_bounds__(256) adjoint_dots_kernel(const T *__restrict__
         const int q1 = min(n, q0 + seg);  // rows [q0, q1); edges (m, m+1) for m in [q0, q1), m + 1 < n
         const long long outer = l0 / inner;
         const size_t base = (size_t)outer * n * inner + (size_t)(l0 - outer * inner);
-        const T *__restrict__ mp = mu + base;
-        const T *__restrict__ yp = y + base;
+        const T *mp = mu + base;
+        const T *yp = y + base;
         // rebuilt ends, read by the segments holding rows 0, n-2 and n-1
         EndFix fx[VEC];
         bool any_fix = false;
@@ -648,9 +648,8 @@ __global__ void __launch_bounds__(256) adjoint_dots_kernel(const T *__restrict__
 // SC: the substrate count when a compile-time constant (1 to 3: part of a
 // vector's neighbours are its own elements), 0 otherwise.
 template <typename T, int VW, int SC>
-__global__ void __launch_bounds__(256) adjoint_dots_flat_kernel(const T *__restrict__ mu, const T *__restrict__ y,
-                                                                DirFaces<T> dir, long long N, int W, int steps,
-                                                                AdjTerms t) {
+__global__ void __launch_bounds__(256) adjoint_dots_flat_kernel(const T *mu, const T *y, DirFaces<T> dir,
+                                                                long long N, int W, int steps, AdjTerms t) {
     __shared__ double s0[256 * VW], s1[256 * VW];
     const int S = SC > 0 ? SC : dir.S, nz = dir.nz, L = nz * S;
     const int tid = threadIdx.x;
@@ -680,8 +679,8 @@ __global__ void __launch_bounds__(256) adjoint_dots_flat_kernel(const T *__restr
                 y1[u] = y0[u + SC < VW ? u + SC : u];
             } else {
                 const long long x = min(e0 + u + S, N - 1);
-                m1[u] = (double)__ldg(mu + x);
-                y1[u] = (double)__ldg(y + x);
+                m1[u] = (double)mu[x];
+                y1[u] = (double)y[x];
             }
         }
         const long long row = N <= 0xffffffffLL ? (long long)((unsigned)e0 / (unsigned)L) : e0 / L;
@@ -883,9 +882,9 @@ __global__ void adjoint_mask_kernel(T *f, DirFaces<T> dir) {
 
 // Agents' update of a recomputed step, keeping the pre-agent values v.
 template <typename T>
-__global__ void cells_keep_kernel(T *__restrict__ f, int S, int n_occ, const int *__restrict__ seg_start,
+__global__ void cells_keep_kernel(T *f, int S, int n_occ, const int *__restrict__ seg_start,
                                   const int *__restrict__ seg_voxel, const T *__restrict__ t1, const T *__restrict__ t2,
-                                  T *__restrict__ vkeep) {
+                                  T *vkeep) {
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= (long long)n_occ * S) return;
     pdl_wait();
@@ -913,10 +912,10 @@ __global__ void cells_keep_kernel(T *__restrict__ f, int S, int n_occ, const int
 // mu_x, and its active-face entries are masked here: the next step's leading
 // Dirichlet overwrote those voxels.
 template <typename T>
-__global__ void cells_adjoint_kernel(T *__restrict__ lam, T *__restrict__ w, const T *__restrict__ vkeep, int S,
-                                     int n_occ, const int *__restrict__ seg_start, const int *__restrict__ seg_voxel,
-                                     const T *__restrict__ t1, const T *__restrict__ t2, double *__restrict__ gt1,
-                                     double *__restrict__ gt2, DirFaces<T> dir) {
+__global__ void cells_adjoint_kernel(T *lam, T *w, const T *vkeep, int S, int n_occ,
+                                     const int *__restrict__ seg_start, const int *__restrict__ seg_voxel,
+                                     const T *__restrict__ t1, const T *__restrict__ t2, double *gt1, double *gt2,
+                                     DirFaces<T> dir) {
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= (long long)n_occ * S) return;
     pdl_wait();

@@ -176,14 +176,14 @@ __global__ void gather_constants_kernel(const int *__restrict__ counts, int S, c
 
 // BioFVM_basic_agent.cpp:291-296 for all agents of one voxel, in list order.
 template <typename T>
-__global__ void cells_kernel(T *__restrict__ f, int S, int nz, int Lp, int n_occ, const int *__restrict__ seg_start,
+__global__ void cells_kernel(T *f, int S, int nz, int Lp, int n_occ, const int *__restrict__ seg_start,
                              const int *__restrict__ seg_voxel, const T *__restrict__ t1, const T *__restrict__ t2) {
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= (long long)n_occ * S) return;
     const int s = (int)(e / S), d = (int)(e % S);
     const size_t fe = voxel_elem(seg_voxel[s], d, nz, S, Lp);
     const int a0 = seg_start[s], a1 = seg_start[s + 1];
-    pdl_wait();  // the segments are host-made; the field is the sweep's
+    pdl_wait();  // the segments are complete (bfb_set_agents waits for them); the field is the sweep's
     T x = f[fe];
     for (int a = a0; a < a1; ++a) {
         const size_t q = (size_t)a * S + d;

@@ -46,7 +46,11 @@ int env_check_device_error(::bfb_env_s *env);
 // (CTAs placed, barriers initialised) while this one drains; it must call
 // pdl_wait before it touches what earlier kernels wrote, which returns once
 // they have completed and their writes are visible. Every kernel launched
-// this way waits, so completion stays transitive along the stream. A kernel
+// this way waits, so completion stays transitive along the stream. What an
+// earlier kernel may still be writing when such a kernel starts is not read-only
+// for its lifetime: pointers to it carry no __restrict__ and are not read by
+// __ldg, either of which would let the compiler move a load above the wait or
+// take it from the read-only path. A kernel
 // lets the next one in (pdl_launch_dependents) when its tile is solved, not
 // when it starts: waiting CTAs hold the shared memory that other envs' kernels
 // beside them could use (three 101x103x99 x 5 FP64 envs stepped side by side

@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(256) bulk_kernel(T *f, const T *__restrict__ A
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= nvec) return;
     const VT av = __ldg(a + e), bv = __ldg(b + e);
-    pdl_wait();  // the coefficients are host-made; the field is an earlier kernel's
+    pdl_wait();  // the coefficients are complete (bfb_set_bulk waits for them); the field is an earlier kernel's
     r[e] = BulkVec<T>::update(r[e], av, bv, dt);
     pdl_launch_dependents();
 }
