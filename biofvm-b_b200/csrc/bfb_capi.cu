@@ -372,12 +372,44 @@ int env_tile_plan(bfb_env_s *env, int elem, int Lp, StridedGeom *gx, StridedGeom
 }
 
 static void drop_graph(bfb_env_s *env) {
-    if (env->graph_exec) cudaGraphExecDestroy(env->graph_exec);
-    env->graph_exec = nullptr;
+    for (cudaGraphExec_t &g : env->graphs) {
+        if (g) cudaGraphExecDestroy(g);
+        g = nullptr;
+    }
     env->graph_flags = -1;
 }
 
-constexpr int kGraphSteps = 8;  // steps per graph of bfb_simulate
+// cudaSuccess when the stream is idle, cudaErrorNotReady when it is not; also
+// while another stream of the caller's is being captured
+static cudaError_t query_stream(cudaStream_t s) {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const cudaError_t q = cudaStreamQuery(s);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (q == cudaErrorNotReady) (void)cudaGetLastError();  // not an error: later launches check for their own
+    return q;
+}
+
+// env->graphs[steps], captured from the env's stream when it is not there yet
+static int make_graph(bfb_env_s *env, double dt, int flags, int steps) {
+    if (env->graphs[steps]) return BFB_OK;
+    cudaGraph_t graph = nullptr;
+    BFB_CUDA(cudaStreamBeginCapture(env->stream, cudaStreamCaptureModeThreadLocal));
+    const int cst = run_steps_any(env, dt, steps, flags, env->stream);
+    cudaError_t e = cudaStreamEndCapture(env->stream, &graph);
+    if (cst) {
+        if (graph) cudaGraphDestroy(graph);
+        return cst;
+    }
+    if (e != cudaSuccess) return cuda_fail(e, "cudaStreamEndCapture");
+    e = cudaGraphInstantiate(&env->graphs[steps], graph, 0);
+    cudaGraphDestroy(graph);
+    if (e != cudaSuccess) {
+        env->graphs[steps] = nullptr;
+        return cuda_fail(e, "cudaGraphInstantiate");
+    }
+    return BFB_OK;
+}
 
 static int check_env(bfb_env_s *env) {
     if (!env) return fail(BFB_ERR_INVALID_ARG, "null bfb_env");
@@ -957,14 +989,13 @@ BFB_API int bfb_simulate(bfb_env env, double dt, int n_steps, int flags) {
     BFB_CUDA(cudaStreamIsCapturing(env->stream, &capturing));
     if (capturing != cudaStreamCaptureStatusNone)  // a graph launch cannot be captured
         return cuda_fail(cudaErrorIllegalState, "bfb_simulate on a capturing stream (BFB_OPT_USE_GRAPHS is on)");
-    // Steps are issued as kernel launches at first, and as replays of a graph
-    // of kGraphSteps of them once the same steps keep coming. Launched one
-    // after the other, the steps' kernels overlap each other's launch
-    // latency, which they do not from one graph to the next (64^3 x 4 FP32:
-    // 18.8 us a step launched, 20.1 as one graph a step), and a first call
-    // pays no capture (10 steps on a new 75^3 env: 473 us against 600). A
-    // graph of many steps keeps the overlap inside it and takes the launch
-    // work off the host.
+    // Steps are issued as kernel launches at first, and as replays of graphs
+    // once the same steps keep coming. Launched one after the other, the steps'
+    // kernels overlap each other's launch latency, which they do not from one
+    // graph to the next (64^3 x 4 FP32: 18.8 us a step launched, 20.1 as one
+    // graph a step), and a first call pays no capture (10 steps on a new 75^3
+    // env: 473 us against 600). A graph of many steps keeps the overlap inside
+    // it and takes the launch work off the host.
     if (env->graph_flags != flags || env->graph_dt != dt || env->graph_epoch != env->epoch) {
         drop_graph(env);
         env->graph_flags = flags;
@@ -972,28 +1003,32 @@ BFB_API int bfb_simulate(bfb_env env, double dt, int n_steps, int flags) {
         env->graph_epoch = env->epoch;
         env->graph_seen = 0;
     }
+    constexpr int kGraphSteps = bfb_env_s::kGraphSteps;
+    env->graph_seen = (int)std::min<long long>((long long)env->graph_seen + n_steps, 1 << 30);
+    if (env->graph_seen < 4 * kGraphSteps) return run_steps_any(env, dt, n_steps, flags, env->stream);
     int left = n_steps;
-    if (!env->graph_exec) {
-        const long long seen = (long long)env->graph_seen + n_steps;
-        env->graph_seen = (int)std::min<long long>(seen, 1 << 30);
-        if (seen < 4 * kGraphSteps || n_steps < kGraphSteps) return run_steps_any(env, dt, n_steps, flags, env->stream);
-        cudaGraph_t graph = nullptr;
-        BFB_CUDA(cudaStreamBeginCapture(env->stream, cudaStreamCaptureModeThreadLocal));
-        int cst = run_steps_any(env, dt, kGraphSteps, flags, env->stream);
-        cudaError_t e = cudaStreamEndCapture(env->stream, &graph);
-        if (cst) {
-            if (graph) cudaGraphDestroy(graph);
-            return cst;
+    if (n_steps >= kGraphSteps) {
+        if ((st = make_graph(env, dt, flags, kGraphSteps))) return st;
+        for (; left >= kGraphSteps; left -= kGraphSteps)
+            BFB_CUDA(cudaGraphLaunch(env->graphs[kGraphSteps], env->stream));
+    } else {
+        // A short call on a busy stream is launched: the device is behind, and
+        // the kernels overlap those of the call before (32x30x28 x 2 FP64, one
+        // step a call: 24.9 us a step; 30.7 as one graph a call without the
+        // overlap inside it). On an idle stream the host is late, because it
+        // waits between calls or steps many envs in turn, and one graph launch
+        // costs it 2 us against 10 to 20 for three to five kernels: 16 such envs
+        // with faces and agents in turn 9.1 -> 4.0 us a call, 16^3 11.1 -> 3.9,
+        // 64^3 x 4 FP32 9.7 -> 7.0; a call that is waited for 34.6 -> 33.8, one
+        // of five steps 135 -> 129. Few envs in turn settle between the two.
+        const cudaError_t q = query_stream(env->stream);
+        if (q == cudaSuccess) {
+            if ((st = make_graph(env, dt, flags, n_steps))) return st;
+            BFB_CUDA(cudaGraphLaunch(env->graphs[n_steps], env->stream));
+            return BFB_OK;
         }
-        if (e != cudaSuccess) return cuda_fail(e, "cudaStreamEndCapture");
-        e = cudaGraphInstantiate(&env->graph_exec, graph, 0);
-        cudaGraphDestroy(graph);
-        if (e != cudaSuccess) {
-            env->graph_exec = nullptr;
-            return cuda_fail(e, "cudaGraphInstantiate");
-        }
+        if (q != cudaErrorNotReady) return cuda_fail(q, "cudaStreamQuery");
     }
-    for (; left >= kGraphSteps; left -= kGraphSteps) BFB_CUDA(cudaGraphLaunch(env->graph_exec, env->stream));
     return run_steps_any(env, dt, left, flags, env->stream);
 }
 

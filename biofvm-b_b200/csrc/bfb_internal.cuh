@@ -197,11 +197,13 @@ struct bfb_env_s {
 
     // CUDA graph of bfb_simulate
     int use_graphs = 1;
-    cudaGraphExec_t graph_exec = nullptr;
+    // bfb_simulate's graphs: graphs[n] replays n steps (made when first needed)
+    static constexpr int kGraphSteps = 8;
+    cudaGraphExec_t graphs[kGraphSteps + 1] = {};
     int graph_flags = -1;
     double graph_dt = 0;
-    uint64_t graph_epoch = 0;            // the epoch the graph (or its count of steps) belongs to
-    int graph_seen = 0;                  // steps issued by launches since then
+    uint64_t graph_epoch = 0;            // the epoch the graphs (and the count of steps) belong to
+    int graph_seen = 0;                  // steps asked for since then
     uint64_t epoch = 1;                  // bumps whenever captured state changes
 
     bfb::SweepTuning tuning;

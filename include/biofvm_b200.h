@@ -61,7 +61,10 @@ typedef struct bfb_env_s *bfb_env;
 #define BFB_OPT_FREEZE_FACTORS 1 /* 1 (default): Thomas factors are computed on the first step
                                     and kept, as BioFVM_parallel.cpp:714,913 does; 0: recomputed
                                     whenever dt differs from the cached one */
-#define BFB_OPT_USE_GRAPHS 2     /* 1 (default): bfb_simulate replays a captured CUDA graph once the same steps keep coming */
+#define BFB_OPT_USE_GRAPHS 2     /* 1 (default): bfb_simulate replays captured CUDA graphs once the same steps
+                                  * have come 32 times: of eight steps in calls of eight or more, of the whole
+                                  * call in shorter ones that find the stream idle (on a busy stream their
+                                  * kernels are launched, overlapping the call before) */
 #define BFB_OPT_USE_TMA 3        /* 1 (default): sweeps move data with the TMA engine where the
                                     grid's row pitch allows; 0: cp.async kernels everywhere */
 

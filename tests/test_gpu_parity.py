@@ -8,6 +8,7 @@ FP32 is compared with a stated relative L-inf tolerance.
 """
 from __future__ import annotations
 
+import time
 from pathlib import Path
 
 import numpy as np
@@ -257,6 +258,69 @@ def test_simulate_launches_and_graph_agree(bfb, oracle, rng, calls):
             if cells:
                 want = oracle.cells_step(want, vox, t1, t2)
         assert np.array_equal(env.get_field(), want)
+
+
+@pytest.mark.parametrize("wait", [True, False])
+def test_simulate_short_calls_keep_agreeing(bfb, oracle, rng, wait):
+    """Calls of one to seven steps after many of the same: graphs of that many steps where the
+    stream is idle, launches where it is busy, and eight-step graphs in between; also when the
+    agents are set anew and the flags change."""
+    shape, S = (9, 12, 10), 2
+    D, lam = log_uniform(rng, 1e2, 1e5, S), log_uniform(rng, 1e-3, 1.0, S)
+    want = rng.random((*shape, S))
+    env = make_env(bfb, want, D, lam, bfb.FP64)
+    box = (0.0, 0.0, 0.0, *(20.0 * v for v in shape))
+    env.simulate(0.01, 40)
+    want = oracle.lod_steps(want, 0.01, 20.0, D, lam, 40)
+    for n_agents in (0, 50, 20):
+        flags, vox = bfb.STEP_DIFFUSION, None
+        if n_agents:
+            flags |= bfb.STEP_CELLS
+            pos = rng.random((n_agents, 3)) * np.array(shape) * 20.0
+            vol = np.full(n_agents, 500.0)
+            sec, upt, sat = log_uniform(rng, 1e-2, 10.0, (3, n_agents, S))
+            env.set_agents(pos, vol, sec, upt, sat, 0.01)
+            vox = oracle.bin_agents(pos, box, 20.0, shape)
+            t1, t2 = oracle.agent_constants(0.01, 20.0, vol, sec, upt, sat)
+        total = 0
+        for n in (20, 12, 1, 1, 2, 7, 3, 4, 5, 6, 11, 1, 7, 3):
+            if wait:
+                env.synchronize()
+            env.simulate(0.01, n, flags)
+            total += n
+        for _ in range(total):
+            want = oracle.lod_steps(want, 0.01, 20.0, D, lam, 1)
+            if vox is not None:
+                want = oracle.cells_step(want, vox, t1, t2)
+        assert np.array_equal(env.get_field(), want)
+
+
+def test_one_step_calls_of_many_envs_are_not_bound_by_launches(bfb, rng):
+    """Sixteen small envs stepped in turn by one-step calls: a call is one graph launch where the
+    stream is idle, so the round takes well under the time that launching every kernel takes
+    (measured 2.3 against 12 us a call; half is asked for)."""
+    shape, S = (16, 16, 16), 1
+    envs = [make_env(bfb, rng.random((*shape, S)), np.full(S, 1e4), np.full(S, 0.1), bfb.FP32) for _ in range(16)]
+
+    def seconds():
+        best = 1e9
+        for _ in range(5):
+            t0 = time.perf_counter()
+            for _ in range(100):
+                for e in envs:
+                    e.simulate(0.01, 1)
+            for e in envs:
+                e.synchronize()
+            best = min(best, time.perf_counter() - t0)
+        return best
+
+    seconds()
+    graphs = seconds()
+    for e in envs:
+        e.set_option(bfb.OPT_USE_GRAPHS, 0)
+    seconds()
+    launches = seconds()
+    assert graphs < 0.5 * launches, (graphs, launches)
 
 
 @pytest.mark.parametrize("sizes", [(1, 300, 0, 40), (257, 256, 255, 1200, 7)])
