@@ -476,7 +476,7 @@ __global__ void __launch_bounds__(128, 1) adjoint_solve_contig_pipe_kernel(Sweep
 // mu.Lap y, sum_(m < n-1) (mu_m - mu_(m+1)) (y_m - y_(m+1)), with y's face
 // ends rebuilt (EndFix). Each line is cut into segments of `seg` rows; one
 // thread walks one segment of VEC adjacent lines (rows [s*seg, s*seg + seg)
-// and the edge out of its last row) with 16-byte loads when VEC > 1.
+// and the edge out of its last row) with 16-byte loads.
 // Element m of line l is at (l / inner) * n * inner + (l % inner) + m * inner;
 // thread g takes lines VEC * (g % (nlines / VEC)) + [0, VEC) and segment
 // g / (nlines / VEC), so consecutive threads read consecutive addresses on
@@ -487,19 +487,15 @@ __global__ void __launch_bounds__(128, 1) adjoint_solve_contig_pipe_kernel(Sweep
 // ---------------------------------------------------------------------------
 template <typename T, int VEC>
 __device__ __forceinline__ void load_vec(const T *p, double (&o)[VEC]) {
-    if constexpr (VEC == 1) {
-        o[0] = (double)p[0];
+    if constexpr (sizeof(T) == 8) {
+        static_assert(VEC == 2, "FP64 rows are read 2 at a time");
+        const double2 v = *reinterpret_cast<const double2 *>(p);
+        o[0] = v.x;
+        o[1] = v.y;
     } else {
-        if constexpr (sizeof(T) == 8) {
-            static_assert(VEC == 2, "FP64 rows are read 2 at a time");
-            const double2 v = *reinterpret_cast<const double2 *>(p);
-            o[0] = v.x;
-            o[1] = v.y;
-        } else {
-            static_assert(VEC == 4, "FP32 rows are read 4 at a time");
-            const float4 v = *reinterpret_cast<const float4 *>(p);
-            o[0] = v.x, o[1] = v.y, o[2] = v.z, o[3] = v.w;
-        }
+        static_assert(VEC == 4, "FP32 rows are read 4 at a time");
+        const float4 v = *reinterpret_cast<const float4 *>(p);
+        o[0] = v.x, o[1] = v.y, o[2] = v.z, o[3] = v.w;
     }
 }
 
@@ -639,14 +635,14 @@ __global__ void __launch_bounds__(256) adjoint_dots_kernel(const T *mu, const T 
 }
 
 // The same sums along z where the substrates of a voxel are not whole vectors
-// (adjoint_dots_kernel would walk each line alone, two or three adjacent values
-// per warp load): the packed field is read straight through in 16-byte vectors
-// (the last elements one by one), a voxel's neighbour being the element S
-// further on, which L1 holds. Thread t takes positions VW*t + q*W, W a multiple
+// but a row of nz of them is (so nz >= 2, and vectors lie in one row): the packed
+// field is read straight through in 16-byte vectors, a voxel's neighbour being
+// the element S further on, which L1 holds; line by line, a load would have two
+// or three adjacent values. Thread t takes positions VW*t + q*W, W a multiple
 // of S, so each vector lane's substrate is fixed; the block adds its lanes per
 // substrate in a fixed tree.
 // SC: the substrate count when a compile-time constant (1 to 3: part of a
-// vector's neighbours are its own elements), 0 otherwise.
+// vector's neighbours may be its own elements), 0 otherwise.
 template <typename T, int VW, int SC>
 __global__ void __launch_bounds__(256) adjoint_dots_flat_kernel(const T *mu, const T *y, DirFaces<T> dir,
                                                                 long long N, int W, int steps, AdjTerms t) {
@@ -662,16 +658,8 @@ __global__ void __launch_bounds__(256) adjoint_dots_flat_kernel(const T *mu, con
     for (int q = 0; q < steps; ++q, e0 += W) {
         if (VW * tid >= W || e0 >= N) break;
         double m0[VW], y0[VW], m1[VW], y1[VW];
-        if (e0 + VW <= N) {
-            load_vec<T, VW>(mu + e0, m0);
-            load_vec<T, VW>(y + e0, y0);
-        } else {
-#pragma unroll
-            for (int u = 0; u < VW; ++u) {
-                m0[u] = e0 + u < N ? (double)mu[e0 + u] : 0.0;
-                y0[u] = e0 + u < N ? (double)y[e0 + u] : 0.0;
-            }
-        }
+        load_vec<T, VW>(mu + e0, m0);
+        load_vec<T, VW>(y + e0, y0);
 #pragma unroll
         for (int u = 0; u < VW; ++u) {
             if (SC > 0 && u + SC < VW) {
@@ -687,24 +675,19 @@ __global__ void __launch_bounds__(256) adjoint_dots_flat_kernel(const T *mu, con
         const int r = (int)(e0 - row * L);
 #pragma unroll
         for (int u = 0; u < VW; ++u) {
-            int re = r + u;  // element of its row; rows shorter than a vector may lie in between
-            long long rw = row;
-            while (re >= L) {
-                re -= L;
-                ++rw;
-            }
+            const int re = r + u;  // element of its row
             const bool first = re < S, last = re >= L - S, before = re >= L - 2 * S && !last;
             double yu = y0[u];
-            if (dir.any && (first || last || before) && e0 + u < N) {  // y rebuilt at the ends on active z faces
+            if (dir.any && (first || last || before)) {  // y rebuilt at the ends on active z faces
                 const int d = re % S;
                 const unsigned msk = dir.mask[d];
                 if (msk & 48u) {
-                    const T *yp = y + (size_t)rw * L;
-                    const int i = (int)(rw / dir.ny), j = (int)(rw - (long long)i * dir.ny);
+                    const T *yp = y + (size_t)row * L;
+                    const int i = (int)(row / dir.ny), j = (int)(row - (long long)i * dir.ny);
                     EndFix fx;
                     fx.make(msk & 16u, msk & 32u, nz, t.c1[d], t.c2[d], (double)dir_value(dir, i, j, 0, d),
-                            (double)dir_value(dir, i, j, nz - 1, d), nz > 1 ? (double)yp[S + d] : 0.0,
-                            nz > 1 ? (double)yp[(size_t)(nz - 2) * S + d] : 0.0);
+                            (double)dir_value(dir, i, j, nz - 1, d), (double)yp[S + d],
+                            (double)yp[(size_t)(nz - 2) * S + d]);
                     if (first && fx.lo) yu = fx.y0;
                     if (last && fx.hi) yu = fx.yn;
                     if (before && fx.hi) y1[u] = fx.yn;
@@ -1066,7 +1049,9 @@ struct Adjoint {
         return launch_contig<T>(a, warps, env->use_tma && env->tuning.tma[2], st, env->tuning.chunks[2]);
     }
 
-    // the sums of one sweep over the stored y and the new mu
+    // the sums of one sweep over the stored y and the new mu, after a bulk-copy
+    // solve, so the axis' lines are whole 16-byte vectors apart (x, y) or rows of
+    // whole vectors (z, S <= 32)
     // lines per thread (16-byte loads) and rows per thread in the sums kernel
     // (measured at 256^3 x 8 FP32: 4 lines x 64 rows beats 1 x 64, 4 x 16 and
     // 4 x 32, and ties with 4 x 128)
@@ -1077,17 +1062,17 @@ struct Adjoint {
     // (128^3 x 2 FP32: 64 blocks of 64 rows 22.6 us, 512 of 8 17.0)
     int dots_seg(int axis) const {
         const int n = axis_len(env, axis);
-        const long long groups = (long long)env->N / n / dots_vec(axis);
-        int seg = dots_vec(axis) == kVec ? kDotSeg : 64;
+        const long long groups = (long long)env->N / n / kVec;
+        int seg = kDotSeg;
         while (seg > 8 && groups * ((n + seg - 1) / seg) < 296LL * dots_threads()) seg /= 2;
         return seg;
     }
     // z where a voxel's substrates are not whole vectors: adjoint_dots_flat_kernel, W positions a step
-    bool dots_flat(int axis) const { return axis == 2 && S % kVec != 0 && S <= 256; }
+    bool dots_flat(int axis) const { return axis == 2 && kc > 0 && S % kVec != 0; }
     int dots_flat_width() const {
         int l = S;
         while (l % kVec) l += S;
-        return l <= kVec * 256 ? (kVec * 256) / l * l : 0;
+        return (kVec * 256) / l * l;
     }
     int dots_flat_steps() const {  // per block
         const long long w = dots_flat_width(), all = (env->N + w - 1) / w;
@@ -1102,32 +1087,31 @@ struct Adjoint {
     long long axis_inner(int axis) const {
         return axis == 0 ? (long long)env->ny * env->nz * S : (axis == 1 ? (long long)env->nz * S : S);
     }
-    int dots_vec(int axis) const { return axis_inner(axis) % kVec == 0 ? kVec : 1; }
     long long dots_blocks(int axis) const {
         const int n = axis_len(env, axis);
-        if (dots_flat(axis) && dots_flat_width()) {
+        if (dots_flat(axis)) {
             const long long w = (long long)dots_flat_width() * dots_flat_steps();
             return (env->N + w - 1) / w;
         }
         const int sg = dots_seg(axis);
-        const long long work = (long long)env->N / n / dots_vec(axis) * ((n + sg - 1) / sg);
+        const long long work = (long long)env->N / n / kVec * ((n + sg - 1) / sg);
         return (work + dots_threads() - 1) / dots_threads();
     }
     int dots(int axis, const SweepArgs<T> &a, const T *mu, const T *y, const AdjTerms &t) {
         const int n = axis_len(env, axis);
         const long long nlines = (long long)env->N / n;
         const unsigned blocks = (unsigned)dots_blocks(axis);
-        const int seg = dots_seg(axis);
-        if (dots_flat(axis) && dots_flat_width()) {
-            const auto k = S == 1   ? adjoint_dots_flat_kernel<T, kVec, 1>
-                           : S == 2 ? adjoint_dots_flat_kernel<T, kVec, 2>
-                           : S == 3 ? adjoint_dots_flat_kernel<T, kVec, 3>
-                                    : adjoint_dots_flat_kernel<T, kVec, 0>;
+        if (dots_flat(axis)) {
+            auto k = adjoint_dots_flat_kernel<T, kVec, 0>;
+            if (S == 1) k = adjoint_dots_flat_kernel<T, kVec, 1>;
+            if (S == 3) k = adjoint_dots_flat_kernel<T, kVec, 3>;
+            if constexpr (kVec == 4)  // in FP64 two substrates are a whole vector
+                if (S == 2) k = adjoint_dots_flat_kernel<T, kVec, 2>;
             BFB_CUDA(launch_pdl(k, blocks, 256, 0, st, mu, y, a.dir, (long long)env->N,
                                 dots_flat_width(), dots_flat_steps(), t));
         } else {
-            const auto k = dots_vec(axis) == kVec ? adjoint_dots_kernel<T, kVec> : adjoint_dots_kernel<T, 1>;
-            BFB_CUDA(launch_pdl(k, blocks, dots_threads(), 0, st, mu, y, a.dir, axis, n, axis_inner(axis), nlines, seg, t));
+            BFB_CUDA(launch_pdl(adjoint_dots_kernel<T, kVec>, blocks, dots_threads(), 0, st, mu, y, a.dir, axis, n,
+                                axis_inner(axis), nlines, dots_seg(axis), t));
         }
         return BFB_OK;
     }

@@ -129,6 +129,27 @@ def test_adjoint_z_sums_of_odd_substrate_counts(bfb, oracle, shape, S):
     env.close()
 
 
+@pytest.mark.parametrize("shape,S", [((3, 2, 4), 1), ((5, 4, 2), 2), ((6, 3, 4), 3), ((4, 5, 16), 2), ((7, 6, 20), 5),
+                                     ((9, 7, 34), 6), ((40, 33, 8), 7), ((5, 4, 12), 31), ((33, 9, 40), 1)])
+def test_adjoint_fp32_z_sums(bfb, oracle, shape, S):
+    """FP32 rows of whole vectors of four whose substrates are not: each instantiation of the flat
+    z sums, with faces at both ends and several blocks, against the kernels without bulk copies on
+    the same FP32 fields (1e-5: FP32 rounding times a cancellation of up to 100 in the sums) and
+    against the FP64 oracle (1e-3, as the FP32 training gradients)."""
+    rng = np.random.default_rng(1900 + S + shape[2])
+    dt = 0.01
+    env, D, lam, rho0, dirv, ag = _setup(bfb, bfb.FP32, shape, S, rng, dt=dt)
+    w = rng.random(rho0.shape) + 0.5
+    ref = oracle_adjoint(oracle, rho0, w, 3, dt, env.dx, D, lam, dirv, ag)
+    got = _gpu_adjoint(bfb, env, rho0, w, 3, dt, 2, ag)
+    env.set_option(bfb.OPT_USE_TMA, 0)
+    plain = _gpu_adjoint(bfb, env, rho0, w, 3, dt, 2, ag)
+    for k in ("initial", "D", "lambda"):
+        assert _rel(got[k], plain[k]) <= 1e-5, k
+        assert _rel(got[k], ref[k]) <= 1e-3, k
+    env.close()
+
+
 def test_adjoint_is_deterministic(bfb):
     rng = np.random.default_rng(9)
     env, D, lam, rho0, dirv, ag = _setup(bfb, bfb.FP64, (40, 36, 44), 3, rng, n_agents=300)
