@@ -123,7 +123,7 @@ static int tail_start(const std::vector<std::vector<double>> &tabs, int n, int S
 //   FP32: 1/den as a hi+lo pair of floats, c1/den and c rounded once; the
 //         deviation form of the FP32 kernels (bfb_sweeps.cuh) needs no c1.
 static int upload_factors(bfb_env_s *env, Uploads &up, int axis, int n, const std::vector<double> &den,
-                          const std::vector<double> &c, const std::vector<double> &c1) {
+                          const std::vector<double> &c, const std::vector<double> &c1, RecipTable &recips) {
     const int S = env->S;
     const size_t nS = (size_t)n * S;
     std::vector<std::vector<double>> tabs;
@@ -147,14 +147,13 @@ static int upload_factors(bfb_env_s *env, Uploads &up, int axis, int n, const st
     const int m0 = tail_start(tabs, n, S);
     int fast = 0;
     if (env->precision == BFB_FP64) {
-        std::vector<double> rl(nS, 0.0);
+        const int last = std::min(m0, n - 1);
+        prove_rows(den, tabs[2], S, last, recips);
         fast = kFastTail | kFastHead;
-        for (int m = 1; m <= std::min(m0, n - 1); ++m)
-            for (int d = 0; d < S; ++d) {
-                const size_t q = (size_t)m * S + d;
-                if (!two_term_reciprocal(den[q], tabs[2][q], &rl[q])) fast &= ~(m < m0 ? kFastHead : kFastTail);
-            }
-        tabs.push_back(rl);
+        for (int m = 1; m <= last; ++m)
+            for (int d = 0; d < S; ++d)
+                if (recips.state[(size_t)m * S + d] != RecipTable::kProven) fast &= ~(m < m0 ? kFastHead : kFastTail);
+        tabs.push_back(recips.lo);
     }
     std::vector<double> flat, tail(4 * (size_t)S, 0.0);
     flat.reserve(4 * nS);
@@ -189,12 +188,13 @@ static int ensure_factors(bfb_env_s *env, double dt) {
     if (env->factors_valid && (env->freeze_factors || env->factor_dt == dt)) return BFB_OK;
     const int ns[3] = {env->nx_global ? env->nx_global : env->nx, env->ny, env->nz};  // a slab: the whole x line
     std::vector<double> den, c, c1;
+    RecipTable recips;
     // the factor tables are only read by kernels on env->stream
     BFB_CUDA(cudaStreamSynchronize(env->stream));
     Uploads up(env->stream);
     for (int a = 0; a < 3; ++a) {
         axis_factors(ns[a], env->S, dt, env->dx, env->D.data(), env->lambda.data(), den, c, c1);
-        int st = upload_factors(env, up, a, ns[a], den, c, c1);
+        int st = upload_factors(env, up, a, ns[a], den, c, c1, recips);
         if (st) return st;
     }
     int st = upload_table(env, up, env->c1, std::move(c1));

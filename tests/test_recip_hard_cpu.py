@@ -74,3 +74,14 @@ def test_search_visits_exactly_the_hard_numerators(driver, P):
             if 0 < min(rem, Y - rem) <= 4:
                 want.add(X)
         assert got == want, Y
+
+
+def test_equal_axes_are_proven_once(driver):
+    """An axis tries only the divisors that the axis before has not: none on an equal one, a last
+    row (3 substrates) on a shorter one, the rows beyond on a longer one; the results are those
+    of a proof on its own."""
+    r = subprocess.run([str(driver), "axes", "40", "40", "25", "90"], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stderr
+    rows = [tuple(map(int, ln.split())) for ln in r.stdout.splitlines()]
+    assert all(same for _, _, same in rows)
+    assert [shared for _, shared, _ in rows] == [3 * 39, 0, 3, 3 * (89 - 23)]
