@@ -220,7 +220,11 @@ struct AgentScratch {
 // agents once per mechanics step; allocating and freeing seventeen arrays on
 // each call (every cudaFree waits for the device) took most of a call's time:
 // 40,000 agents x 4 substrates 4.3 -> 0.41 ms a call, 100,000 x 8 12 -> 1.3,
-// now bound by the rates crossing the host link from pageable memory.
+// now bound by the rates crossing the host link from pageable memory. An empty
+// set gives the block back, and so does one that needs under a quarter of a
+// block of more than kAgentBlockKeep bytes (a smaller one is not worth the
+// wait for the device that freeing it takes).
+constexpr size_t kAgentBlockKeep = 16 << 20;
 int agents_layout(bfb_env_s *env, int n, bool rates, AgentScratch *w) {
     const size_t N = (size_t)n, nS = N * env->S;
     int end_bit = 1;
@@ -264,7 +268,7 @@ int agents_layout(bfb_env_s *env, int n, bool rates, AgentScratch *w) {
         take((char **)&w->tmp, std::max(w->sort_bytes, w->select_bytes));
     };
     lay();
-    if (off > env->ag_ws_bytes) {
+    if (off > env->ag_ws_bytes || (env->ag_ws_bytes > kAgentBlockKeep && off < env->ag_ws_bytes / 4)) {
         const size_t want = off + off / 4;  // agents divide
         agents_free(env);
         BFB_CUDA(cudaMalloc(&env->ag_ws, want));
@@ -315,6 +319,7 @@ int agents_quiesce(bfb_env_s *env) {
 int agents_build(bfb_env_s *env, int n, const double *pos, const double *volume, const double *sec,
                  const double *upt, const double *sat, const uint8_t *active, double dt) {
     int st = agents_quiesce(env);
+    if (!st && n == 0) agents_free(env);
     if (st || n == 0) return st;
     const int S = env->S;
     const size_t nS = (size_t)n * S;
@@ -360,6 +365,7 @@ int agents_build(bfb_env_s *env, int n, const double *pos, const double *volume,
 int agents_build_constants(bfb_env_s *env, int n, const int *voxel, const double *t1, const double *t2,
                            const uint8_t *active) {
     int st = agents_quiesce(env);
+    if (!st && n == 0) agents_free(env);
     if (st || n == 0) return st;
     const int S = env->S;
     const size_t nS = (size_t)n * S;

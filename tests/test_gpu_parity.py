@@ -352,6 +352,26 @@ def test_agents_set_again_and_again(bfb, oracle, rng, sizes):
         env.set_agent_constants(np.array([0, 6 * 5 * 7]), np.zeros((2, S)), np.ones((2, S)))
 
 
+def test_agent_memory_is_given_back(bfb, rng):
+    """A large agent set's device memory goes back to the device with the next empty set, and with
+    a set of a small part of its size."""
+    torch = pytest.importorskip("torch")
+    shape, S, n = (8, 9, 10), 2, 1_000_000
+    env = make_env(bfb, rng.random((*shape, S)), np.ones(S), np.ones(S), bfb.FP64)
+
+    def put(k):
+        env.set_agents(rng.random((k, 3)) * 160.0, np.ones(k), *np.ones((3, k, S)), 0.01)
+        return torch.cuda.mem_get_info()[0]
+
+    put(n)  # the kernels are loaded
+    none = put(0)
+    large = put(n)
+    assert large < none - (64 << 20)
+    assert put(10) > none - (16 << 20)
+    assert put(n) < none - (64 << 20)
+    assert put(0) > none - (4 << 20)
+
+
 def test_agents_random_fp64_and_fp32(bfb, oracle, rng):
     shape, S = (20, 18, 16), 3
     dx, dt = 20.0, 0.01
