@@ -305,10 +305,9 @@ int agents_finish(bfb_env_s *env, Uploads &up, const AgentScratch &w) {
     return BFB_OK;
 }
 
-// No kernel may still read the agent arrays: the env's own stream is idle
-// (bfb_set_agents waits for it), a batch's streams may not be.
-int agents_quiesce(bfb_env_s *env) {
-    if (env->batched) BFB_CUDA(cudaDeviceSynchronize());
+// Drops the agent set once no kernel reads it any more.
+int agents_drop(bfb_env_s *env) {
+    if (int st = env_quiesce(env)) return st;
     env->n_agents = env->n_occ = env->n_active = 0;
     env->rates_known = false;
     return BFB_OK;
@@ -318,7 +317,7 @@ int agents_quiesce(bfb_env_s *env) {
 
 int agents_build(bfb_env_s *env, int n, const double *pos, const double *volume, const double *sec,
                  const double *upt, const double *sat, const uint8_t *active, double dt) {
-    int st = agents_quiesce(env);
+    int st = agents_drop(env);
     if (!st && n == 0) agents_free(env);
     if (st || n == 0) return st;
     const int S = env->S;
@@ -364,7 +363,7 @@ int agents_build(bfb_env_s *env, int n, const double *pos, const double *volume,
 
 int agents_build_constants(bfb_env_s *env, int n, const int *voxel, const double *t1, const double *t2,
                            const uint8_t *active) {
-    int st = agents_quiesce(env);
+    int st = agents_drop(env);
     if (!st && n == 0) agents_free(env);
     if (st || n == 0) return st;
     const int S = env->S;

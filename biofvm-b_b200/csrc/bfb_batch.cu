@@ -378,7 +378,7 @@ struct bfb_batch_s {
     std::vector<std::vector<bfb_env>> chains;
     std::vector<cudaStream_t> chain_streams;
     cudaGraphExec_t graph = nullptr;        // one step
-    cudaGraphExec_t graph_multi = nullptr;  // kMultiSteps steps (both built together)
+    cudaGraphExec_t graph_multi = nullptr;  // kMultiSteps steps
     static constexpr int kMultiSteps = 8;
     int graph_flags = -1;
     double graph_dt = 0;
@@ -911,7 +911,9 @@ BFB_API int bfb_batch_autotune(bfb_batch b, double dt, int flags, int trials, in
     if (!b) return fail(BFB_ERR_INVALID_ARG, "null bfb_batch");
     if (!(dt > 0) || trials < 1) return fail(BFB_ERR_INVALID_ARG, "dt must be > 0 and trials >= 1");
     BFB_CUDA(cudaSetDevice(b->device));
-    // the trial steps advance the fields: keep copies and put them back
+    // the trial steps advance the fields: keep copies and put them back (steps
+    // that the batch has not finished yet come first)
+    BFB_CUDA(cudaStreamSynchronize(b->stream));
     std::vector<void *> saved(b->n, nullptr);
     int st = BFB_OK;
     for (int k = 0; k < b->n && !st; ++k) {

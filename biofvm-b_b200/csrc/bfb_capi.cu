@@ -189,8 +189,7 @@ static int ensure_factors(bfb_env_s *env, double dt) {
     const int ns[3] = {env->nx_global ? env->nx_global : env->nx, env->ny, env->nz};  // a slab: the whole x line
     std::vector<double> den, c, c1;
     RecipTable recips;
-    // the factor tables are only read by kernels on env->stream
-    BFB_CUDA(cudaStreamSynchronize(env->stream));
+    if (int st = env_quiesce(env)) return st;
     Uploads up(env->stream);
     for (int a = 0; a < 3; ++a) {
         axis_factors(ns[a], env->S, dt, env->dx, env->D.data(), env->lambda.data(), den, c, c1);
@@ -436,9 +435,10 @@ static int bulk_tabulate(bfb_env_s *env, const double *Sr, const double *T, cons
         BFB_CUDA(cudaMalloc(&env->bulkB, env->elem * env->Np));
         BFB_CUDA(cudaMemsetAsync(env->bulkB, 0, env->elem * env->Np, env->stream));
     }
-    BFB_CUDA(cudaStreamSynchronize(env->stream));
+    int st = env_quiesce(env);
+    if (st) return st;
     Uploads up(env->stream);
-    int st = upload_pitched_table(env, up, env->bulkA, std::move(A));
+    st = upload_pitched_table(env, up, env->bulkA, std::move(A));
     if (!st) st = upload_pitched_table(env, up, env->bulkB, std::move(B));
     if (st) return st;
     BFB_CUDA(up.wait());
@@ -448,6 +448,12 @@ static int bulk_tabulate(bfb_env_s *env, const double *Sr, const double *T, cons
 }  // namespace bfb
 
 using namespace bfb;
+
+int bfb::env_quiesce(bfb_env_s *env) {
+    BFB_CUDA(cudaStreamSynchronize(env->stream));
+    if (env->batched) BFB_CUDA(cudaDeviceSynchronize());
+    return BFB_OK;
+}
 
 // The device error flag is sticky: once a kernel's bounded wait ran out, the
 // env's field is not trustworthy and every later synchronize reports it.
@@ -822,7 +828,7 @@ static int dirichlet_install(bfb_env_s *env, std::vector<double> *faces_host /* 
             BFB_CUDA(cudaMalloc(&env->faces[f], env->elem * fsz[f] * S));
             BFB_CUDA(cudaMemsetAsync(env->faces[f], 0, env->elem * fsz[f] * S, env->stream));
         }
-    BFB_CUDA(cudaStreamSynchronize(env->stream));
+    if (int st = env_quiesce(env)) return st;
     Uploads up(env->stream);
     if (faces_host)
         for (int f = 0; f < 6; ++f) {
@@ -935,7 +941,6 @@ BFB_API int bfb_set_agents(bfb_env env, int n, const double *pos, const double *
     if (n < 0) return fail(BFB_ERR_INVALID_ARG, "n < 0");
     if (n > 0 && (!pos || !volume || !secretion || !uptake || !saturation))
         return fail(BFB_ERR_INVALID_ARG, "agent arrays must not be NULL");
-    BFB_CUDA(cudaStreamSynchronize(env->stream));
     st = agents_build(env, n, pos, volume, secretion, uptake, saturation, active, dt);
     if (!st) env->agent_dt = dt;
     env->epoch++;
@@ -948,7 +953,6 @@ BFB_API int bfb_set_agent_constants(bfb_env env, int n, const int *voxel, const 
     if (st) return st;
     if (n < 0) return fail(BFB_ERR_INVALID_ARG, "n < 0");
     if (n > 0 && (!voxel || !temp1 || !temp2)) return fail(BFB_ERR_INVALID_ARG, "agent arrays must not be NULL");
-    BFB_CUDA(cudaStreamSynchronize(env->stream));
     st = agents_build_constants(env, n, voxel, temp1, temp2, active);
     env->epoch++;
     return st;

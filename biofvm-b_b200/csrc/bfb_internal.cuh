@@ -36,6 +36,12 @@ int cuda_fail(cudaError_t e, const char *what);
 // not trustworthy), BFB_OK otherwise.
 int env_check_device_error(::bfb_env_s *env);
 
+// Waits until no kernel reads the env's device arrays (factors, faces, bulk
+// coefficients, agents) any more, before they are overwritten in place: for the
+// env's stream, and where a batch was made over the env, whose steps run on
+// streams of its own, for the device.
+int env_quiesce(::bfb_env_s *env);
+
 #define BFB_CUDA(call)                                        \
     do {                                                      \
         cudaError_t _e = (call);                              \
@@ -189,7 +195,7 @@ struct bfb_env_s {
     void *ag_ws = nullptr;               // the block holding all of the above (agents_layout)
     size_t ag_ws_bytes = 0;
     int ag_end_bit = 1;                  // key bits of the voxel sort
-    bool batched = false;                // a batch was made over this env: its streams may read the agents
+    bool batched = false;                // a batch was made over this env: its streams may read its arrays
 
     // scratch for reductions
     double *partials = nullptr;

@@ -280,7 +280,9 @@ BFB_API int bfb_checksum(bfb_env env, double *out);
  *     launches them), one independent branch per env of the step's graph,
  *     so the hardware schedules the envs' CTAs side by side.
  * The batch references the envs; they must outlive it, and their own settings
- * (coefficients, Dirichlet, agents) are the ones used.
+ * (coefficients, Dirichlet, agents) are the ones used. They may be changed
+ * between calls without waiting: the change waits for the batch's steps. Field
+ * transfers and an env's own steps do not; call bfb_batch_synchronize first.
  * bfb_batch_simulate_loop runs the same steps as one bfb_simulate call per
  * env (the per-instance launch loop). Not in the reference, which runs one
  * Microenvironment per MPI job. */

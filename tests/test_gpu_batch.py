@@ -247,3 +247,42 @@ def test_ensemble_256_batch_vs_loop_and_fp64_check(bfb):
           f"per-instance loop {t_loop * 1e3:.3f} ms/step ({vs / t_loop:.3e}); "
           f"FP32 vs FP64 rel Linf on 8 envs: max {max(errs):.2e}")
     assert max(errs) <= 1e-5
+
+
+@pytest.mark.parametrize("mode", ["staged", "persistent", "graph"])
+@pytest.mark.parametrize("n_envs", [5, 40])
+def test_settings_change_while_the_batch_runs(bfb, oracle, mode, n_envs):
+    """Agents (fewer, more, none), coefficients and faces set anew on a batch's envs right after a
+    call that has not been waited for, and the autotuner on steps in flight: every call uses the
+    settings of its own time; bit for bit."""
+    dt = 0.01
+    rng = np.random.default_rng(500 + n_envs)
+    made = [make_instance(bfb, rng, 10, 30 if n_envs < 10 else 14, 200, bfb.FP64, dt) for _ in range(n_envs)]
+    specs, envs = (list(v) for v in zip(*made))
+    batch = bfb.Batch(envs)
+    batch.set_mode(MODES[mode])
+    want = [sp["rho0"] for sp in specs]
+    flags = bfb.STEP_DIFFUSION | bfb.STEP_CELLS
+    for q, (steps, n_agents) in enumerate([(40, None), (24, 30), (9, 700), (17, 0), (8, 100)]):
+        if n_agents is not None:
+            for k in range(0, n_envs, 2):
+                sp = specs[k]
+                sp["pos"] = rng.random((n_agents, 3)) * np.array(sp["shape"]) * 20.0
+                sp["vol"] = np.full(n_agents, 500.0)
+                sp["sec"], sp["upt"], sp["sat"] = log_uniform(rng, 1e-2, 10.0, (3, n_agents, sp["S"]))
+                envs[k].set_agents(sp["pos"], sp["vol"], sp["sec"], sp["upt"], sp["sat"], dt)
+            for k in range(1, n_envs, 2):
+                sp = specs[k]
+                if q % 2:
+                    sp["D"] = log_uniform(rng, 1e2, 1e5, sp["S"])
+                    envs[k].set_coefficients(sp["D"], sp["lam"])
+                else:
+                    sp["fm"] = np.zeros((6, sp["S"]), np.uint8)
+                    sp["fm"][q, 0] = 1
+                    envs[k].set_dirichlet_uniform(sp["act"], np.full(sp["S"], 38.0), face_mask=sp["fm"])
+        batch.simulate(dt, steps, flags)
+        for k, sp in enumerate(specs):
+            want[k] = oracle_run(oracle, dict(sp, rho0=want[k]), dt, steps)
+    batch.autotune(dt, flags, trials=1)  # its copies wait for the steps above
+    for sp, env, w in zip(specs, envs, want):
+        assert np.array_equal(env.get_field(), w), sp["shape"]
