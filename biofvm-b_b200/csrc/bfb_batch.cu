@@ -408,6 +408,10 @@ using namespace bfb;
 //    48 of 24-80                334 -> 297    48 of 32-160   1146 -> 982
 //   256 of 16-48                642 -> 614   256 of 32-160   5745 -> 5530
 constexpr long long kOwnChainBytes = 1 << 20;
+static bool has_own_chain(const bfb_batch_s *b, int k) {
+    const bfb_env_s *e = b->envs[k];
+    return b->n <= bfb_batch_s::kMaxChains || e->Np * e->elem >= kOwnChainBytes;
+}
 
 template <typename T>
 static int batch_upload(bfb_batch_s *b, double dt) {
@@ -486,14 +490,13 @@ static int batch_upload(bfb_batch_s *b, double dt) {
     // whose smallest tile needs more than half the class's largest (at most 4
     // classes per group and path)
     auto warp_of = [](size_t bytes) { return (int)((128 + bytes + 127) / 128 * 128); };
-    // Envs of kOwnChainBytes or more are left out of the shared launches
-    // (group -1) and spread over chains of their own kernels in the same way.
+    // Envs with chains of their own are left out of the shared launches (group
+    // -1) and spread over the chains in the same way.
     std::vector<int> group(b->n, 0);
     {
         auto work = [&](int k) { return (double)b->envs[k]->N; };
         std::vector<int> order, own;
-        for (int k = 0; k < b->n; ++k)
-            (b->n <= bfb_batch_s::kMaxChains || b->envs[k]->Np * (long long)eb >= kOwnChainBytes ? own : order).push_back(k);
+        for (int k = 0; k < b->n; ++k) (has_own_chain(b, k) ? own : order).push_back(k);
         auto larger = [&](int x, int y) { return work(x) > work(y); };
         std::stable_sort(order.begin(), order.end(), larger);
         std::stable_sort(own.begin(), own.end(), larger);
@@ -933,12 +936,18 @@ BFB_API int bfb_batch_autotune(bfb_batch b, double dt, int flags, int trials, in
     const int old_w = b->warps, old_t = b->tiles_per_item, old_m = b->mode;
     int best_w = old_w, best_t = old_t, best_m = old_m;
     double best = -1.0;
-    // staged: warps per CTA only (tiles per item is a persistent-mode knob)
+    // staged: warps per CTA only (tiles per item is a persistent-mode knob), and
+    // only where envs share stage launches: an env's own kernels have its own shape
     struct Shape {
         int mode, w, tpi;
     };
     std::vector<Shape> shapes;
-    for (int w : {1, 2, 4}) shapes.push_back({BFB_BATCH_MODE_STAGED, w, old_t});
+    bool shared = false;
+    for (int k = 0; k < b->n; ++k) shared = shared || !has_own_chain(b, k);
+    if (shared)
+        for (int w : {1, 2, 4}) shapes.push_back({BFB_BATCH_MODE_STAGED, w, old_t});
+    else
+        shapes.push_back({BFB_BATCH_MODE_STAGED, old_w, old_t});
     for (int w : {1, 2, 4})
         for (int tpi : {1, 2, 4, 8}) shapes.push_back({BFB_BATCH_MODE_PERSISTENT, w, tpi});
     shapes.push_back({BFB_BATCH_MODE_GRAPH, old_w, old_t});

@@ -272,8 +272,8 @@ BFB_API int bfb_checksum(bfb_env env, double *out);
  * graph, in one of three modes:
  *   BFB_BATCH_MODE_STAGED (default): one launch per stage (x, y, z sweeps,
  *     agents), each a flat grid over the envs' tiles, one warp per tile;
- *     larger envs, and all envs of a small batch, are stepped by their own
- *     kernels beside them;
+ *     envs with a field of 1 MB or more, and all envs of a batch of at most
+ *     32, are stepped by their own kernels beside them;
  *   BFB_BATCH_MODE_PERSISTENT: ONE persistent kernel launch per step whose
  *     warps pull (env, stage, tile) work items from a device queue;
  *   BFB_BATCH_MODE_GRAPH: every env's own step kernels (as bfb_simulate
@@ -287,7 +287,8 @@ BFB_API int bfb_checksum(bfb_env env, double *out);
  * env (the per-instance launch loop). Not in the reference, which runs one
  * Microenvironment per MPI job. */
 typedef struct bfb_batch_s *bfb_batch;
-#define BFB_BATCH_OPT_WARPS_PER_CTA 1   /* 1..4, default 1 */
+#define BFB_BATCH_OPT_WARPS_PER_CTA 1   /* 1..4, default 1: of the staged mode's shared launches and the persistent
+                                           kernel; an env's own kernels have the env's own shape (bfb_set_tuning) */
 #define BFB_BATCH_OPT_TILES_PER_ITEM 2  /* warp tiles per queue item (persistent mode), 1..64, default 2 */
 #define BFB_BATCH_OPT_MODE 3            /* BFB_BATCH_MODE_STAGED (default), _PERSISTENT or _GRAPH */
 #define BFB_BATCH_MODE_PERSISTENT 0
@@ -304,8 +305,9 @@ BFB_API int bfb_batch_simulate_loop(bfb_batch batch, double dt, int n_steps, int
  * instead (NULL: back to its own), e.g. to time them with events there. */
 BFB_API int bfb_batch_set_stream(bfb_batch batch, void *cuda_stream);
 BFB_API int bfb_batch_synchronize(bfb_batch batch);
-/* Times bfb_batch_simulate in the staged mode with warps per CTA {1, 2, 4},
- * in the persistent mode with warps per CTA {1, 2, 4} x tiles per item
+/* Times bfb_batch_simulate in the staged mode with warps per CTA {1, 2, 4}
+ * (once, with the present setting, where every env is stepped by its own
+ * kernels), in the persistent mode with warps per CTA {1, 2, 4} x tiles per item
  * {1, 2, 4, 8} and in the graph mode (8 warm steps and 8*`trials` timed
  * steps each, CUDA events; bfb_batch_simulate replays 8 steps per graph
  * launch while at least 8 remain), keeps the fastest and returns it in

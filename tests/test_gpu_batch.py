@@ -249,6 +249,83 @@ def test_ensemble_256_batch_vs_loop_and_fp64_check(bfb):
     assert max(errs) <= 1e-5
 
 
+def shared_stage_envs(bfb, kind, prec, dt, n=36):
+    """More envs than a batch steps by their own kernels, each under 1 MB, so that all share the
+    staged mode's launches: ragged shapes, shapes whose rows suit TMA on every axis, some with
+    more than 32 substrates, or some without bulk copies (the cp.async tiles of both widths)."""
+    rng = np.random.default_rng(sum(map(ord, kind)))
+    made = []
+    for k in range(n):
+        if kind == "aligned":
+            shape, S = tuple(int(v) * 8 for v in rng.integers(1, 4, 3)), int(rng.choice([2, 4]))
+        elif kind == "wide" and k % 3 == 0:
+            shape, S = tuple(int(v) for v in rng.integers(2, 9, 3)), int(rng.choice([33, 40]))
+        else:
+            shape, S = tuple(int(v) for v in rng.integers(1, 25, 3)), int(rng.integers(1, 7))
+        na = int(rng.integers(0, 200))
+        sec, upt, sat = log_uniform(rng, 1e-2, 10.0, (3, na, S))
+        fm = np.zeros((6, S), np.uint8)
+        fm[:, 0] = [1, 1, 0, 1, 1, 0]
+        act = np.zeros(S, np.uint8)
+        act[0] = 1
+        box = np.array(shape) * 20.0
+        spec = dict(shape=shape, S=S, D=log_uniform(rng, 1e2, 1e5, S), lam=log_uniform(rng, 1e-3, 1.0, S),
+                    rho0=rng.random((*shape, S)), fm=fm, act=act, pos=rng.random((na, 3)) * box,
+                    vol=np.full(na, 500.0), sec=sec, upt=upt, sat=sat, box=(0, 0, 0, *box))
+        env = build(bfb, spec, prec, dt)
+        if kind == "plain" and k % 2:
+            env.set_option(bfb.OPT_USE_TMA, 0)
+        made.append((spec, env))
+    return tuple(zip(*made))
+
+
+@pytest.mark.parametrize("kind", ["ragged", "aligned", "wide", "plain"])
+@pytest.mark.parametrize("warps", [1, 2, 4])
+def test_shared_stages_fp64_bitexact(bfb, oracle, kind, warps):
+    """The staged mode's shared launches on every kind of tile: FP64 against the oracle."""
+    dt, steps = 0.01, 3
+    specs, envs = shared_stage_envs(bfb, kind, bfb.FP64, dt)
+    batch = bfb.Batch(envs)
+    batch.set_mode(bfb.BATCH_MODE_STAGED)
+    batch.set_warps(warps)
+    batch.simulate(dt, steps, bfb.STEP_DIFFUSION | bfb.STEP_CELLS)
+    batch.synchronize()
+    for spec, env in zip(specs, envs):
+        assert np.array_equal(env.get_field(), oracle_run(oracle, spec, dt, steps)), (spec["shape"], spec["S"])
+
+
+@pytest.mark.parametrize("kind", ["ragged", "aligned", "wide", "plain"])
+@pytest.mark.parametrize("warps", [1, 4])
+def test_shared_stages_fp32_equal_the_loop(bfb, kind, warps):
+    """The same in FP32, bit for bit against one env at a time; nine steps (both graphs)."""
+    dt, steps = 0.01, 9
+    _, envs = shared_stage_envs(bfb, kind, bfb.FP32, dt)
+    _, alone = shared_stage_envs(bfb, kind, bfb.FP32, dt)
+    batch = bfb.Batch(envs)
+    batch.set_mode(bfb.BATCH_MODE_STAGED)
+    batch.set_warps(warps)
+    batch.simulate(dt, steps, bfb.STEP_DIFFUSION | bfb.STEP_CELLS)
+    batch.synchronize()
+    for eb, el in zip(envs, alone):
+        el.simulate(dt, steps, bfb.STEP_DIFFUSION | bfb.STEP_CELLS)
+        el.synchronize()
+        assert np.array_equal(eb.get_field_raw(), el.get_field_raw()), eb.shape
+
+
+def test_batch_autotune_of_own_kernels_keeps_the_warps(bfb):
+    """Where every env is stepped by its own kernels the staged mode has one shape: the autotuner
+    does not choose among equal ones, so a staged choice keeps the setting that has no effect."""
+    rng = np.random.default_rng(32)
+    dt = 0.01
+    _, envs = zip(*[make_aligned_instance(bfb, rng, bfb.FP32, dt, 50) for _ in range(3)])
+    batch = bfb.Batch(envs)
+    for _ in range(8):
+        batch.set_warps(3)
+        batch.set_mode(bfb.BATCH_MODE_STAGED)
+        (w, _), _ = batch.autotune(dt, bfb.STEP_DIFFUSION | bfb.STEP_CELLS, trials=1)
+        assert batch.mode != bfb.BATCH_MODE_STAGED or w == 3
+
+
 @pytest.mark.parametrize("mode", ["staged", "persistent", "graph"])
 @pytest.mark.parametrize("n_envs", [5, 40])
 def test_settings_change_while_the_batch_runs(bfb, oracle, mode, n_envs):
