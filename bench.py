@@ -8,7 +8,7 @@ lambda log-uniform in [1e2, 1e5] / [1e-3, 1] (seeded), U[0,1) field, no
 Dirichlet, no agents -- the configuration the FP32 >= 70 % HBM-roofline
 target is quoted on. Metric: voxel*substrate updates per second per LOD step
 (V*S*K / t). A "step" is one full LOD step (x, y and z Thomas sweeps with the
-fused Dirichlet), replayed from a CUDA graph. The 537 MB FP32 field is larger
+fused Dirichlet), issued by bfb_simulate. The 537 MB FP32 field is larger
 than the 126 MB L2, so no flush is needed between steps.
 
 Multi-GPU: the path does not shard (one grid per GPU); N ranks run N
