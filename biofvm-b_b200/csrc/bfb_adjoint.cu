@@ -952,7 +952,7 @@ __global__ void agent_rates_adjoint_kernel(int n_active, int S, const int *__res
 namespace bfb {
 int env_prepare_step(bfb_env_s *env, double dt, int flags);
 template <typename T>
-SweepArgs<T> env_sweep_args(bfb_env_s *env, int axis);
+SweepArgs<T> env_sweep_args(bfb_env_s *env, int axis, double dt);
 int env_tile_plan(bfb_env_s *env, int elem, int Lp, StridedGeom *gx, StridedGeom *gy, ContigGeom *gz, int vb16[3]);
 }  // namespace bfb
 
@@ -1008,6 +1008,7 @@ void opt_in_all() {
 template <typename T>
 struct Adjoint {
     bfb_env_s *env = nullptr;
+    double dt = 0;
     cudaStream_t st = nullptr;
     int S = 0;
     StridedGeom gx, gy;
@@ -1029,7 +1030,7 @@ struct Adjoint {
     }
     // the env's sweep arguments over packed workspace buffers
     SweepArgs<T> args(int axis) const {
-        SweepArgs<T> a = env_sweep_args<T>(env, axis);
+        SweepArgs<T> a = env_sweep_args<T>(env, axis, dt);
         a.Lp = env->nz * S;
         return a;
     }
@@ -1176,6 +1177,7 @@ int adjoint_run(bfb_env_s *env, double dt, int n_steps, int flags, int K, const 
     if (rc) return rc;
     Adjoint<T> A;
     A.env = env;
+    A.dt = dt;
     A.st = st;
     A.sums = gD || gL;
     A.S = S;
@@ -1341,7 +1343,7 @@ int adjoint_run(bfb_env_s *env, double dt, int n_steps, int flags, int K, const 
     BFB_CUDA(cudaMemcpyAsync(lam.p, dL_dfinal, fb, cudaMemcpyDeviceToDevice, st));
 
     // ---- reverse, segment by segment
-    const DirFaces<T> dirf = env_sweep_args<T>(env, 0).dir;
+    const DirFaces<T> dirf = env_sweep_args<T>(env, 0, dt).dir;
     Buf *pl = &lam, *pm = &mu;
     for (int s = nseg - 1; s >= 0; --s) {
         const int len = s == nseg - 1 ? last_len : K;

@@ -389,7 +389,7 @@ namespace bfb {
 // from bfb_capi.cu
 int env_prepare_step(bfb_env_s *env, double dt, int flags);
 template <typename T>
-SweepArgs<T> env_sweep_args(bfb_env_s *env, int axis);
+SweepArgs<T> env_sweep_args(bfb_env_s *env, int axis, double dt);
 int env_tile_plan(bfb_env_s *env, int elem, int Lp, StridedGeom *gx, StridedGeom *gy, ContigGeom *gz, int vb16[3]);
 int env_run_steps(bfb_env_s *env, double dt, int n, int flags, cudaStream_t s);
 }  // namespace bfb
@@ -414,7 +414,7 @@ static bool has_own_chain(const bfb_batch_s *b, int k) {
 }
 
 template <typename T>
-static int batch_upload(bfb_batch_s *b) {
+static int batch_upload(bfb_batch_s *b, double dt) {
     std::vector<BatchInst<T>> inst(b->n);
     std::vector<CUtensorMap> maps(2 * (size_t)b->n);
     std::vector<int> prefix(4 * (size_t)(b->n + 1), 0), tpre(4 * (size_t)(b->n + 1), 0), perm(4 * (size_t)b->n);
@@ -426,7 +426,7 @@ static int batch_upload(bfb_batch_s *b) {
     for (int k = 0; k < b->n; ++k) {
         bfb_env_s *e = b->envs[k];
         BatchInst<T> &I = inst[k];
-        for (int a = 0; a < 3; ++a) I.ax[a] = env_sweep_args<T>(e, a);
+        for (int a = 0; a < 3; ++a) I.ax[a] = env_sweep_args<T>(e, a, dt);
         int st = env_tile_plan(e, sizeof(T), e->Lp, &I.gx, &I.gy, &I.gz, I.vb16);
         if (st) return st;
         I.tiles[0] = I.gx.n_slabs * I.gx.ncb;
@@ -886,8 +886,8 @@ BFB_API int bfb_batch_simulate(bfb_batch b, double dt, int n_steps, int flags) {
     if (changed || (!b->graph && !b->graph_multi)) {
         batch_drop_graph(b);
         int st = b->mode == BFB_BATCH_MODE_GRAPH ? BFB_OK  // the envs' own launches need no tables
-                 : b->precision == BFB_FP64     ? batch_upload<double>(b)
-                                                : batch_upload<float>(b);
+                 : b->precision == BFB_FP64     ? batch_upload<double>(b, dt)
+                                                : batch_upload<float>(b, dt);
         if (st) return st;
         for (bfb_env e : b->envs) BFB_CUDA(cudaStreamSynchronize(e->stream));
         b->graph_flags = flags;

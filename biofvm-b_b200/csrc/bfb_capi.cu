@@ -216,7 +216,7 @@ static int ensure_factors(bfb_env_s *env, double dt) {
 }
 
 template <typename T>
-static SweepArgs<T> make_args(bfb_env_s *env, int axis) {
+static SweepArgs<T> make_args(bfb_env_s *env, int axis, bool bulk, double dt) {
     SweepArgs<T> a;
     a.f = static_cast<T *>(env->field);
     a.fo = a.f;
@@ -246,16 +246,12 @@ static SweepArgs<T> make_args(bfb_env_s *env, int axis) {
     a.dir.nz = env->nz;
     a.dir.S = env->S;
     a.dir.any = env->dir_any;
+    a.bulk.A = static_cast<const T *>(env->bulkA);
+    a.bulk.B = static_cast<const T *>(env->bulkB);
+    a.bulk.dt = (T)dt;
+    a.bulk.on = bulk && env->bulk_on;
     a.err = env->d_err;
     return a;
-}
-
-// The bulk update, where the env has bulk terms.
-template <typename T>
-static int launch_bulk_env(bfb_env_s *env, double dt, cudaStream_t s) {
-    if (!env->bulk_on) return BFB_OK;
-    const BulkTerms<T> b{static_cast<const T *>(env->bulkA), static_cast<const T *>(env->bulkB), (T)dt};
-    return launch_bulk<T>(static_cast<T *>(env->field), b, env->Np, s);
 }
 
 static const CUtensorMap *tma_map(bfb_env_s *env, int axis) {
@@ -277,8 +273,8 @@ static void encode_field_maps(bfb_env_s *env) {
 }
 
 template <typename T>
-static int launch_strided_env(bfb_env_s *env, int axis, cudaStream_t s) {
-    const SweepArgs<T> a = make_args<T>(env, axis);
+static int launch_strided_env(bfb_env_s *env, int axis, double dt, cudaStream_t s) {
+    const SweepArgs<T> a = make_args<T>(env, axis, false, dt);
     if constexpr (sizeof(T) == 8) {  // the tensor-memory tiles where the tuning asks for them
         if (env->use_tma && env->tuning.tma[axis] == 2 && env->tmem_ok[axis]) {
             const int st = launch_strided_tmem(a, strided_geometry(a, axis), &env->tmem_map[axis],
@@ -297,13 +293,13 @@ static int refuse_slab(const bfb_env_s *env) {
 }
 
 template <typename T>
-static int run_diffusion(bfb_env_s *env, cudaStream_t s) {
+static int run_diffusion(bfb_env_s *env, double dt, cudaStream_t s) {
     if (int st = refuse_slab(env)) return st;
-    int st = launch_strided_env<T>(env, 0, s);
+    int st = launch_strided_env<T>(env, 0, dt, s);
     if (st) return st;
-    st = launch_strided_env<T>(env, 1, s);
+    st = launch_strided_env<T>(env, 1, dt, s);
     if (st) return st;
-    return launch_contig<T>(make_args<T>(env, 2), env->tuning.warps[2],
+    return launch_contig<T>(make_args<T>(env, 2, false, dt), env->tuning.warps[2],
                             env->use_tma != 0 && env->tuning.tma[2] != 0, s, env->tuning.chunks[2]);
 }
 
@@ -311,8 +307,8 @@ template <typename T>
 static int run_steps(bfb_env_s *env, double dt, int n, int flags, cudaStream_t s) {
     for (int q = 0; q < n; ++q) {
         int st = BFB_OK;
-        if (flags & BFB_STEP_BULK) st = launch_bulk_env<T>(env, dt, s);
-        if (!st && (flags & BFB_STEP_DIFFUSION)) st = run_diffusion<T>(env, s);
+        if (flags & BFB_STEP_BULK) st = launch_bulk<T>(make_args<T>(env, 0, true, dt), env->Np, s);
+        if (!st && (flags & BFB_STEP_DIFFUSION)) st = run_diffusion<T>(env, dt, s);
         if (st) return st;
         if (flags & BFB_STEP_CELLS) {
             st = launch_cells(env, s);
@@ -336,11 +332,11 @@ int env_prepare_step(bfb_env_s *env, double dt, int flags) {
 }
 
 template <typename T>
-SweepArgs<T> env_sweep_args(bfb_env_s *env, int axis) {
-    return make_args<T>(env, axis);
+SweepArgs<T> env_sweep_args(bfb_env_s *env, int axis, double dt) {
+    return make_args<T>(env, axis, false, dt);
 }
-template SweepArgs<double> env_sweep_args<double>(bfb_env_s *, int);
-template SweepArgs<float> env_sweep_args<float>(bfb_env_s *, int);
+template SweepArgs<double> env_sweep_args<double>(bfb_env_s *, int, double);
+template SweepArgs<float> env_sweep_args<float>(bfb_env_s *, int, double);
 
 // One or more steps of the env on stream s, as bfb_simulate issues them (the
 // batch's graph mode captures these per env).
@@ -902,8 +898,8 @@ BFB_API int bfb_set_dirichlet_uniform(bfb_env env, const double *value_per_subst
 BFB_API int bfb_apply_dirichlet(bfb_env env) {
     int st = check_env(env);
     if (st) return st;
-    st = env->precision == BFB_FP64 ? launch_dirichlet<double>(make_args<double>(env, 0), env->stream)
-                                    : launch_dirichlet<float>(make_args<float>(env, 0), env->stream);
+    st = env->precision == BFB_FP64 ? launch_dirichlet<double>(make_args<double>(env, 0, false, 0), env->stream)
+                                    : launch_dirichlet<float>(make_args<float>(env, 0, false, 0), env->stream);
     return st;
 }
 
@@ -1141,7 +1137,7 @@ static int time_candidates(bfb_env_s *env, double dt, int trials, void *scratch,
             for (int warps : {1, 2, 4}) {
                 for (int chunks : {2, 4, 8}) {
                     if (!tma && chunks != kChunks) continue;  // the cp.async tiles have a fixed stage count
-                    SweepArgs<T> a = make_args<T>(env, axis);
+                    SweepArgs<T> a = make_args<T>(env, axis, false, dt);
                     a.fo = static_cast<T *>(scratch);
                     CUtensorMap mi, mo;
                     int ci = 0, co = 0;
@@ -1237,22 +1233,23 @@ BFB_API int bfb_profile_steps(bfb_env env, double dt, int n_steps, int flags, do
         const bool fp64 = env->precision == BFB_FP64;
         if (flags & BFB_STEP_BULK)
             st = phase_ms(3, [&] {
-                return fp64 ? launch_bulk_env<double>(env, dt, s) : launch_bulk_env<float>(env, dt, s);
+                return fp64 ? launch_bulk<double>(make_args<double>(env, 0, true, dt), env->Np, s)
+                            : launch_bulk<float>(make_args<float>(env, 0, true, dt), env->Np, s);
             });
         if (!st && (flags & BFB_STEP_DIFFUSION)) {
             st = phase_ms(0, [&] {
-                return fp64 ? launch_strided_env<double>(env, 0, s) : launch_strided_env<float>(env, 0, s);
+                return fp64 ? launch_strided_env<double>(env, 0, dt, s) : launch_strided_env<float>(env, 0, dt, s);
             });
             if (!st)
                 st = phase_ms(1, [&] {
-                    return fp64 ? launch_strided_env<double>(env, 1, s) : launch_strided_env<float>(env, 1, s);
+                    return fp64 ? launch_strided_env<double>(env, 1, dt, s) : launch_strided_env<float>(env, 1, dt, s);
                 });
             if (!st)
                 st = phase_ms(2, [&] {
                     const bool tz = env->use_tma != 0 && env->tuning.tma[2] != 0;
-                    return fp64 ? launch_contig<double>(make_args<double>(env, 2), env->tuning.warps[2], tz,
+                    return fp64 ? launch_contig<double>(make_args<double>(env, 2, false, dt), env->tuning.warps[2], tz,
                                                         s, env->tuning.chunks[2])
-                                : launch_contig<float>(make_args<float>(env, 2), env->tuning.warps[2], tz, s,
+                                : launch_contig<float>(make_args<float>(env, 2, false, dt), env->tuning.warps[2], tz, s,
                                                        env->tuning.chunks[2]);
                 });
         }
@@ -1334,7 +1331,7 @@ BFB_API int bfb_slab_x_forward(bfb_env env, double dt, const double *prev_in, do
     if ((st = slab_half_args(env, dt, line0, line1))) return st;
     if (env->x0 > 0 && !prev_in) return fail(BFB_ERR_INVALID_ARG, "prev_in is NULL past the grid's first plane");
     NvtxRange range("bfb_slab_x_forward");
-    return launch_slab_x_forward(make_args<double>(env, 0), env->x0, env->nx_global, line0, line1,
+    return launch_slab_x_forward(make_args<double>(env, 0, false, dt), env->x0, env->nx_global, line0, line1,
                                  env->x0 > 0 ? prev_in : nullptr, prev_out, env->stream);
 }
 
@@ -1346,7 +1343,7 @@ BFB_API int bfb_slab_x_backward(bfb_env env, double dt, const double *next_in, d
     const bool last = env->x0 + env->nx == env->nx_global;
     if (!last && !next_in) return fail(BFB_ERR_INVALID_ARG, "next_in is NULL before the grid's last plane");
     NvtxRange range("bfb_slab_x_backward");
-    return launch_slab_x_backward(make_args<double>(env, 0), env->x0, env->nx_global, line0, line1,
+    return launch_slab_x_backward(make_args<double>(env, 0, false, dt), env->x0, env->nx_global, line0, line1,
                                   last ? nullptr : next_in, next_out, env->stream);
 }
 
@@ -1355,7 +1352,7 @@ BFB_API int bfb_slab_yz(bfb_env env, double dt) {
     if (st) return st;
     if ((st = slab_half_args(env, dt, 0, 0))) return st;
     NvtxRange range("bfb_slab_yz");
-    if ((st = launch_strided_env<double>(env, 1, env->stream))) return st;
-    return launch_contig<double>(make_args<double>(env, 2), env->tuning.warps[2],
+    if ((st = launch_strided_env<double>(env, 1, dt, env->stream))) return st;
+    return launch_contig<double>(make_args<double>(env, 2, false, dt), env->tuning.warps[2],
                                  env->use_tma != 0 && env->tuning.tma[2] != 0, env->stream, env->tuning.chunks[2]);
 }

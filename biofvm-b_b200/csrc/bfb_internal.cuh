@@ -113,6 +113,7 @@ struct BulkTerms {
     const T *A;
     const T *B;
     T dt;
+    int on;
 };
 
 // Launch shape of the three sweeps, chosen by bfb_autotune or set by

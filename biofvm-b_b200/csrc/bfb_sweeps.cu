@@ -531,10 +531,12 @@ int launch_dirichlet(const SweepArgs<T> &a, cudaStream_t s) {
 }
 
 template <typename T>
-int launch_bulk(T *field, const BulkTerms<T> &b, long long N, cudaStream_t s) {
+int launch_bulk(const SweepArgs<T> &a, long long N, cudaStream_t s) {
+    if (!a.bulk.on) return BFB_OK;
     constexpr int kVec = 16 / (int)sizeof(T);  // the rows are whole 16-byte vectors (bfb_env_s::Lp)
     const long long nvec = N / kVec;
-    BFB_CUDA(launch_pdl(bulk_kernel<T>, (unsigned)((nvec + 255) / 256), 256, 0, s, field, b.A, b.B, b.dt, nvec));
+    BFB_CUDA(launch_pdl(bulk_kernel<T>, (unsigned)((nvec + 255) / 256), 256, 0, s, a.f, a.bulk.A, a.bulk.B, a.bulk.dt,
+                        nvec));
     return BFB_OK;
 }
 
@@ -597,7 +599,7 @@ template int launch_contig<double>(const SweepArgs<double> &, int, bool, cudaStr
 template int launch_contig<float>(const SweepArgs<float> &, int, bool, cudaStream_t, int);
 template int launch_dirichlet<double>(const SweepArgs<double> &, cudaStream_t);
 template int launch_dirichlet<float>(const SweepArgs<float> &, cudaStream_t);
-template int launch_bulk<double>(double *, const BulkTerms<double> &, long long, cudaStream_t);
-template int launch_bulk<float>(float *, const BulkTerms<float> &, long long, cudaStream_t);
+template int launch_bulk<double>(const SweepArgs<double> &, long long, cudaStream_t);
+template int launch_bulk<float>(const SweepArgs<float> &, long long, cudaStream_t);
 
 }  // namespace bfb
