@@ -378,13 +378,19 @@ static void drop_graph(bfb_env_s *env) {
     env->graph_flags = -1;
 }
 
-// cudaSuccess when the stream is idle, cudaErrorNotReady when it is not; also
-// while another stream of the caller's is being captured
-static cudaError_t query_stream(cudaStream_t s) {
+// While the calling thread captures another stream of its own (torch.cuda.graph
+// does so in the global mode), queries and graph instantiation are refused and
+// would break that capture, unless the thread's mode is relaxed around them.
+struct RelaxedCapture {
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    cudaThreadExchangeStreamCaptureMode(&mode);
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// cudaSuccess when the stream is idle, cudaErrorNotReady when it is not
+static cudaError_t query_stream(cudaStream_t s) {
+    const RelaxedCapture relaxed;
     const cudaError_t q = cudaStreamQuery(s);
-    cudaThreadExchangeStreamCaptureMode(&mode);
     if (q == cudaErrorNotReady) (void)cudaGetLastError();  // not an error: later launches check for their own
     return q;
 }
@@ -392,6 +398,7 @@ static cudaError_t query_stream(cudaStream_t s) {
 // env->graphs[steps], captured from the env's stream when it is not there yet
 static int make_graph(bfb_env_s *env, double dt, int flags, int steps) {
     if (env->graphs[steps]) return BFB_OK;
+    const RelaxedCapture relaxed;
     cudaGraph_t graph = nullptr;
     BFB_CUDA(cudaStreamBeginCapture(env->stream, cudaStreamCaptureModeThreadLocal));
     const int cst = run_steps_any(env, dt, steps, flags, env->stream);

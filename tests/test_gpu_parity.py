@@ -295,6 +295,32 @@ def test_simulate_short_calls_keep_agreeing(bfb, oracle, rng, wait):
         assert np.array_equal(env.get_field(), want)
 
 
+@pytest.mark.parametrize("n", [3, 20])
+def test_simulate_while_the_caller_captures_its_own_stream(bfb, oracle, rng, n):
+    """Steps on the env's stream, graphs made among them, while the caller captures another stream
+    in the global mode: both work."""
+    torch = pytest.importorskip("torch")
+    shape, S = (9, 8, 10), 2
+    D, lam = log_uniform(rng, 1e2, 1e5, S), log_uniform(rng, 1e-3, 1.0, S)
+    want = rng.random((*shape, S))
+    env = make_env(bfb, want, D, lam, bfb.FP64)
+    env.simulate(0.01, 7)
+    for _ in range(4):
+        env.simulate(0.01, 7)  # 35 steps in short calls on a busy stream: no graph yet
+    env.synchronize()
+    x = torch.zeros(1000, device="cuda")
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        x.add_(1.0)
+        env.simulate(0.01, n)
+        x.add_(1.0)
+        env.simulate(0.01, n)
+    g.replay()
+    torch.cuda.synchronize()
+    assert float(x.min()) == float(x.max()) == 2.0
+    assert np.array_equal(env.get_field(), oracle.lod_steps(want, 0.01, 20.0, D, lam, 35 + 2 * n))
+
+
 def test_the_call_that_makes_the_graph_hides_it(bfb):
     """A long call whose steps become a graph takes no longer than the next one: the device works
     on launched steps while the graph is captured and instantiated (2 ms, or 7 % of this call)."""
